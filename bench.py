@@ -296,9 +296,8 @@ def wait_probe(moe, steps):
     L.hmoe_probe_read(buf, 1)
     if steps is None:
         return {}
-    names = {0: "mma_thread_waits_for_weights", 1: "mma_thread_waits_for_inputs", 2: "mma_thread_waits_for_free_accumulators",
-             4: "dequant_warp0_waits_for_ring_slot", 10: "dequant_warp15_waits_for_ring_slot", 9: "dequant_warp0_store_fence_arrive",
-             6: "tma_thread_waits_for_ring_slot", 7: "readout_warp_waits_for_tile", 8: "readout_warp_reads_out"}
+    names = {0: "mma_warp_waits_for_converted_stage", 2: "mma_warp_waits_for_free_accumulators", 10: "convert_warp0_waits_for_codes",
+             4: "convert_warp0_waits_for_operand_slot", 9: "convert_warp0_store_and_arrive", 6: "input_warp_waits_for_ring_slot", 7: "readout_warp_waits_for_tile", 8: "readout_warp_reads_out"}
     out = {}
     for k, kernel in ((1, "gate_up"), (0, "down")):
         tot = buf[32 * k + 15]

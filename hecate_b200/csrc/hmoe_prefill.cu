@@ -1,5 +1,5 @@
 // Prefill path of the MoE expert layer (hundreds to tens of thousands of rows), sm_100a: token permutation on the device
-// and two grouped GEMMs on the tcgen05 tensor cores with the int4 weights dequantised on the way into shared memory.
+// and two grouped GEMMs on the tcgen05 tensor cores with the int4 weights converted on the way into tensor memory.
 //
 // Replaces, behind the same operator surface (packed int4 experts in the reference's fragment order, (sel, rw) routing, fp32
 // output added into `out`):
@@ -8,23 +8,24 @@
 //     kernels with no host synchronisation: histogram per 1024-pick chunk, scan + balanced row-block table, stable scatter;
 //   * gather_kernel / p4t_gu_kernel / p4t_gemm_kernel of runtime/tier/moe4/moe4t.cu:113-433 by the kernels below.
 //
-// GEMM orientation: D[channel][pick] = W[channel][k] . X[pick][k]: the weights are the M = 128 operand, the picks of one
-// row block (<= 256, one expert) the N operand, fp32 accumulators in tensor memory. Per 64-column stage:
-//   warps 0-15 read the packed codes of the tile straight from global memory (16 bytes per lane, the stored fragment order),
-//              turn them into fp16 (times the bf16 group scale in the group format) and store them as a K-major,
-//              128-byte-swizzled operand tile (16-byte stores, conflict free); they do nothing else and run ahead of the MMAs
-//              from tile to tile as far as the ring allows;
-//   warp 16    one thread loads the row block's input tile (picks x 64 columns) as 2-D TMA boxes of 64 rows, as many as the block
-//              has picks (128-byte swizzle, rows beyond the array zero-filled);
-//   warp 17    one thread issues tcgen05.mma (M 128, N = picks rounded up to 16, K 16) four times per matrix and commits the
-//              stage back to the producers;
-//   warps 18-21 (down) / 18-25 (gate_up) read the finished sums out of tensor memory (one quarter of the lanes = 32 channels each;
-//              gate_up: two warps per quarter, half the columns each).
-// gate_up keeps two accumulators (gate, up: 2 x 256 columns) over the same input tile and its read-out writes
-// act = SiLU(g) * u * routing weight in fp16; down adds scale * sum into out[token] with coalesced fp32 reductions and keeps two
-// accumulator sets, so a tile's read-out runs under the next tile's MMAs. (Measured on the benchmark with parts of the kernel
-// switched off: the MMA / TMA pipeline alone needs 4.5 ms of a 7.7 ms step, the dequantisation 1.5 ms and the read-outs 1.7 ms
-// when the same warps do both in turn, as an earlier version did; hence the separate warps.)
+// GEMM orientation: D[channel][pick] = W[channel][k] . X[pick][k]: the weights are the M = 128 operand, converted into tensor
+// memory, the picks of one row block (<= 128, one expert) the N operand in shared memory, fp32 accumulators in tensor memory. An
+// item is a row block x two 128-channel tiles (gate and up, or two tiles of down) over the same inputs, so that every input tile
+// feeds two MMA sequences. Per 128-column stage (one scale group):
+//   warp 16    brings the packed codes and scales into shared memory by 1-D bulk copies, five stages ahead;
+//   warps 0-15 in two groups that take the stages in turn: 16 bytes of codes per lane and strip -> fp16 (times the bf16 group scale)
+//              -> tcgen05.st. The stored fragment order of the codes is the row / word order of the 16x256b store, so the weights never
+//              pass through shared memory as fp16: at N <= 128 reading a 128-row operand from shared memory for every MMA, and writing it
+//              there, would ask for more than the 128 bytes per cycle that shared memory gives;
+//   warp 17    brings the stage's inputs (picks x 128 columns) as 2-D TMA boxes of 64 and 16 rows (128-byte swizzle), four stages ahead;
+//   warps 18, 19  issue tcgen05.mma (M 128, N = picks rounded up to 16, K 16), one warp per accumulator, and commit the stage back;
+//   warps 20-27   read the finished sums out of tensor memory (one quarter of the lanes = 32 channels each): gate_up writes
+//              act = SiLU(g) * u * routing weight in fp16; down adds scale * sum into out[token] with coalesced fp32 reductions.
+// What bounds it: up to about 64 picks per expert HBM (every expert's codes once), next to it the conversion (a code costs two of
+// the half-rate instructions, whatever the number of picks); from there on the tensor core at the clock the power cap leaves.
+// Measured (256 experts of 6144 x 2048, us per call before -> after, before: fp16 weights staged through shared memory, row blocks of up
+// to 256 picks): 777 rows, Zipf(1.1) 2872 -> 1735; 2048 rows, fp32 row scales 2753 -> 1821; 8192 rows, Zipf(1.1) 6821 -> 6416 (the last two at
+// 1.45 GHz under the power cap).
 // Blocks are persistent (one per SM) over (row block, channel tile) items, channel tile fastest, so the blocks working at
 // the same time share one input tile and one expert's weights through L2.
 // Every wait is bounded (see mbar_wait); tensor memory is released by the warp that allocated it on every path.
@@ -37,9 +38,9 @@ namespace hmoe {
 namespace {
 
 // Diagnostic build (-DHMOE_PROBE_WAITS): every role adds up the cycles it spends in each of its waits (in registers, one atomic
-// per thread at the end of the kernel); hmoe_probe_read() returns the sums. 32 counters per kernel: 0 / 1 / 2 MMA thread waiting
-// for the weights / the inputs / a free accumulator set, 4 and 10 dequantising warps 0 and 15 waiting for a ring slot, 9 warp 0's
-// stores + fence + arrive, 6 TMA thread waiting for a slot, 7 / 8 first read-out warp waiting for a tile / reading it out, 15
+// per thread at the end of the kernel); hmoe_probe_read() returns the sums. 32 counters per kernel: 0 / 2 first MMA warp waiting
+// for a converted stage (and its inputs) / free accumulators, 10 / 4 converting warp 0 waiting for codes / for its operand slot, 9 its
+// store completion + arrive, 6 input warp waiting for a slot, 7 / 8 first read-out warp waiting for a tile / reading it out, 15
 // the block's lifetime. Not part of the normal build.
 #ifdef HMOE_PROBE_WAITS
 __device__ unsigned long long g_probe[64];
@@ -51,13 +52,10 @@ __device__ unsigned long long g_probe[64];
 #define PROBE_ADD(i)
 #define PROBE_ON(c) false
 #endif
-constexpr int TM = 128, TN = 256, TK = 64;
-constexpr int TB = 64;                          // rows per TMA box of the input tile
-constexpr int NDQ = 16;                         // dequantising warps
-// read-out warps: one per quarter of the tensor-memory lanes in down (whose read-out runs under the next tile's MMAs), two per
-// quarter in gate_up (whose single accumulator set keeps the tensor core waiting until the read-out is done: half the columns each)
-__host__ __device__ constexpr int nepi(int nmat) { return nmat == 2 ? 8 : 4; }
-__host__ __device__ constexpr int pf_threads(int nmat) { return (NDQ + 2 + nepi(nmat)) * 32; }      // warp NDQ: TMA, warp NDQ + 1: MMA, warps NDQ + 2 ..: read-out
+constexpr int TM = 128, TN = 128, TK = 64;
+constexpr int NDQ = 16;                         // converting warps; then codes, inputs, MMA, MMA, read-out
+constexpr int NEPI = 8;
+constexpr int PF_THREADS = (NDQ + 4 + NEPI) * 32;
 constexpr int CHUNK = 1024;                     // picks per permutation block (one warp)
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -204,9 +202,8 @@ __global__ void __launch_bounds__(192) gather_kernel(const void* __restrict__ x,
             for (int k = 0; k < 32; ++k) v[k] = __fmul_rn((float) __float2int_rn(__fmul_rn(v[k], inv)), s);
         }
         const size_t rowlen = act_quant ? 2 * (size_t) H : (size_t) H;       // int8 mode: [hi | lo] halves, code x scale kept to ~22 bits
-        // The 64 columns of a block are stored in the order the weight tiles use (operand_pos): the thread's 32 columns (16-column
-        // steps 2j, 2j + 1 of the block) become, for each q, eight consecutive values = one 16-byte store.
-        const int kb = gi >> 1, j8 = (gi & 1) * 8;
+        // The columns are stored in the order the converted weights use (operand_pos): the thread's two 16-column steps stay in place, and inside
+        // a step the pairs of columns 2q (+ 8 h) become positions 4q + 2h: four consecutive 4-byte pairs = one 16-byte store.
         #pragma unroll
         for (int q = 0; q < 4; ++q)
         {
@@ -214,15 +211,15 @@ __global__ void __launch_bounds__(192) gather_kernel(const void* __restrict__ x,
             #pragma unroll
             for (int i = 0; i < 4; ++i)
             {
-                const int c = (i >> 1) * 16 + (i & 1) * 8 + 2 * q;           // step (i / 2), half (i % 2), columns 2q, 2q + 1
+                const int c = (q >> 1) * 16 + (i & 1) * 8 + 2 * ((q & 1) * 2 + (i >> 1));      // step q / 2, half i % 2, pair 2 (q % 2) + i / 2
                 const __half2 h = __floats2half2_rn(v[c], v[c + 1]);
                 w[i] = *(const uint32_t*) &h;
                 const float2 f = __half22float2(h);
                 const __half2 l = __floats2half2_rn(v[c] - f.x, v[c + 1] - f.y);
                 wl[i] = *(const uint32_t*) &l;
             }
-            *(uint4*) (xg + (size_t) pos * rowlen + kb * 64 + q * 16 + j8) = make_uint4(w[0], w[1], w[2], w[3]);
-            if (act_quant) *(uint4*) (xg + (size_t) pos * rowlen + H + kb * 64 + q * 16 + j8) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+            *(uint4*) (xg + (size_t) pos * rowlen + gi * 32 + q * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+            if (act_quant) *(uint4*) (xg + (size_t) pos * rowlen + H + gi * 32 + q * 8) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
         }
     }
 }
@@ -240,24 +237,35 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr)
 {
     return (uint64_t) ((addr & 0x3FFFFu) >> 4) | ((uint64_t) 1 << 16) | ((uint64_t) (1024 >> 4) << 32) | ((uint64_t) 1 << 46) | ((uint64_t) 2 << 61);
 }
-__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+// A from tensor memory: 128 lanes x 8 words (16 fp16 columns) per instruction
+template <bool FIRST>
+__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc)
 {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+    if (FIRST) asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, 0, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc) : "memory");
+    else asm volatile("{\n .reg .pred p;\n setp.eq.b32 p, 0, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r)
+__device__ __forceinline__ bool elect_one()
 {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-                   "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-                   "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]) : "r"(taddr));
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
 }
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t* r)
+// 16 lanes x 32 words (see the 64-word form below)
+__device__ __forceinline__ void tmem_st_16x256_half(uint32_t taddr, const uint32_t (&r)[16])
 {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63]) : "r"(taddr));
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                   "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+// 16 lanes x 64 words: register 4 i + {0, 1} of lane (g, q) = row g, words 8 i + 2 q, + 1; register 4 i + {2, 3} = row g + 8
+__device__ __forceinline__ void tmem_st_16x256(uint32_t taddr, const uint32_t (&r)[32])
+{
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+                 "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                   "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+                   "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+                   "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r)
 {
@@ -280,7 +288,12 @@ __device__ __forceinline__ void red_add_sys(float* p, float v)
 {
     asm volatile("red.relaxed.sys.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v) : "memory");
 }
-__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ uint2 lds64(uint32_t addr)
+{
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
+}
 
 struct GemmArgs
 {
@@ -288,6 +301,7 @@ struct GemmArgs
     int grouped;              // bf16 scale per 128 columns (else fp32 per row)
     int act_quant;
     int kfold;                // 1, or 2 in the int8 mode: the inputs are [hi | lo] halves over 2 K columns, the weights are walked twice
+    int nsub;                 // sub-blocks of at most TN picks per row block of the table (1; 2 for a caller's table with up to 2 TN picks)
     const int64_t* w0; const int64_t* w1;     // pointer tables of the matrix (gate, up) or (down, -)
     const int64_t* s0; const int64_t* s1;     // scale tables
     const void* sh_w0; const void* sh_w1; const void* sh_s0; const void* sh_s1;   // shared expert (expert id n_local)
@@ -302,43 +316,62 @@ struct GemmArgs
 };
 
 // Column order of the GEMM operands inside every block of 64 columns. The tensor core only needs both operands to agree on
-// which stored position holds which column, so the order is chosen for the weights: a lane (g, q) of the dequantising warps holds,
-// of rows g and g + 8, the columns 16 t + 8 h + 2 q + cc (t = 0..3, h, cc = 0..1) of the block, and these go to positions
-// 16 q + 4 t + 2 h + cc: the lane's sixteen values of a row are contiguous (32 bytes, two 16-byte stores). The gathered inputs
-// and the intermediate activations are written in the same order (gather_kernel, the gate_up read-out).
-__host__ __device__ __forceinline__ int operand_pos(int k) { return ((k >> 1) & 3) * 16 + (k >> 4) * 4 + ((k >> 3) & 1) * 2 + (k & 1); }
+// which stored position holds which column, so the order is chosen for the weights: in the 16 columns of one MMA step a lane (g, q)
+// of a converting warp holds, of rows g and g + 8, the columns 8 h + 2 q + cc (h, cc = 0..1), and the tensor-memory store puts a
+// lane's two words of a row at 32-bit columns 2 q and 2 q + 1, i.e. operand positions 4 q + 2 h + cc. The gathered inputs and the
+// intermediate activations are written in the same order (gather_kernel, the gate_up read-out).
+__host__ __device__ __forceinline__ int operand_pos(int k) { return (k & ~15) + ((k >> 1) & 3) * 4 + ((k >> 3) & 1) * 2 + (k & 1); }
 
-__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
-{
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
-// One 16-row x 64-column strip of packed codes (one 16-byte word per lane) -> 32 fp16 values per lane (a[t] = the four registers
-// of 16-column step t, times the group scale), and their store into the K-major 128-byte-swizzled operand tile as four 16-byte
-// words (conflict free: the eight lanes of a quarter warp hit eight different 16-byte columns). The two halves are separate
-// functions because the conversion is done BEFORE the warp waits for its ring slot: when the slot is released only the four
-// stores stand between the release and the MMA thread's wake-up.
-__device__ __forceinline__ void convert_strip(const uint4& w, uint32_t s_lo, uint32_t s_hi, bool scaled, uint32_t (&a)[4][4])
+// One 16-row x 64-column strip of packed codes (one 16-byte word per lane) -> the four registers of each of its four 16-column
+// steps in the order the tensor-memory store takes them (row g: two words, row g + 8: two words), times the group scale.
+// Logic / shift instructions and half2 arithmetic each run at one warp instruction per two cycles and scheduler, so what counts is
+// the larger of the two counts. UNSCALED: frag_from_codes (5 + 4 per word). SCALED (any scale): a multiply behind it makes that 5 + 8. FUSED:
+// the two codes of the upper byte are instead brought to mantissa bits 6..9 under the exponent of 16, where one fused multiply-add does
+// both steps: (16 + c) s - 24 s, exact because 24 s has at most ten significant bits (s comes from bf16) and (c - 8) s at most eleven: 6 + 6.
+// It needs 31 s inside fp16's range, so a stage with a scale of 2048 or more takes SCALED.
+enum Conv { UNSCALED, SCALED, FUSED };
+template <Conv MODE>
+__device__ __forceinline__ void convert_strip(const uint4& w, uint32_t s_lo, uint32_t s_hi, uint32_t* r)
 {
     const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+    uint32_t o_lo = 0, o_hi = 0;
+    if (MODE == FUSED) { asm("mul.f16x2 %0, %1, %2;" : "=r"(o_lo) : "r"(s_lo), "r"(0xce00ce00u)); asm("mul.f16x2 %0, %1, %2;" : "=r"(o_hi) : "r"(s_hi), "r"(0xce00ce00u)); }     // -24 s
     #pragma unroll
     for (int t = 0; t < 4; ++t)
     {
-        frag_from_codes(ww[t], a[t]);
-        if (scaled)
+        if (MODE != FUSED)
         {
-            asm("mul.f16x2 %0, %0, %1;" : "+r"(a[t][0]) : "r"(s_lo)); asm("mul.f16x2 %0, %0, %1;" : "+r"(a[t][2]) : "r"(s_lo));
-            asm("mul.f16x2 %0, %0, %1;" : "+r"(a[t][1]) : "r"(s_hi)); asm("mul.f16x2 %0, %0, %1;" : "+r"(a[t][3]) : "r"(s_hi));
+            uint32_t a[4];
+            frag_from_codes(ww[t], a);
+            if (MODE == SCALED)
+            {
+                asm("mul.f16x2 %0, %0, %1;" : "+r"(a[0]) : "r"(s_lo)); asm("mul.f16x2 %0, %0, %1;" : "+r"(a[2]) : "r"(s_lo));
+                asm("mul.f16x2 %0, %0, %1;" : "+r"(a[1]) : "r"(s_hi)); asm("mul.f16x2 %0, %0, %1;" : "+r"(a[3]) : "r"(s_hi));
+            }
+            r[4 * t] = a[0]; r[4 * t + 1] = a[2]; r[4 * t + 2] = a[1]; r[4 * t + 3] = a[3];
+        }
+        else
+        {
+            uint32_t lo, hi, lo1, hi1;
+            asm("lop3.b32 %0, %1, 0x000f000f, 0x64006400, 0xea;" : "=r"(lo) : "r"(ww[t]));           // row g, columns 2q (+ 1): 1024 + c
+            asm("lop3.b32 %0, %1, 0x00f000f0, 0x64006400, 0xea;" : "=r"(hi) : "r"(ww[t]));           // row g + 8: 1024 + 16 c
+            asm("lop3.b32 %0, %1, 0x03c003c0, 0x4c004c00, 0xea;" : "=r"(lo1) : "r"(ww[t] >> 2));     // row g, columns 2q + 8 (+ 1): 16 + c
+            asm("lop3.b32 %0, %1, 0x03c003c0, 0x4c004c00, 0xea;" : "=r"(hi1) : "r"(ww[t] >> 6));     // row g + 8
+            asm("sub.f16x2 %0, %0, %1;" : "+r"(lo) : "r"(0x64086408u));
+            asm("fma.rn.f16x2 %0, %0, %1, %2;" : "+r"(hi) : "r"(0x2c002c00u), "r"(0xd480d480u));
+            asm("mul.f16x2 %0, %1, %2;" : "=r"(r[4 * t]) : "r"(lo), "r"(s_lo));
+            asm("mul.f16x2 %0, %1, %2;" : "=r"(r[4 * t + 2]) : "r"(hi), "r"(s_hi));
+            asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r[4 * t + 1]) : "r"(lo1), "r"(s_lo), "r"(o_lo));
+            asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r[4 * t + 3]) : "r"(hi1), "r"(s_hi), "r"(o_hi));
         }
     }
 }
-// row0 = shared address of the lane's row g in the strip's first 8-row group; c0, c1 = byte offsets of its two 16-byte columns
-__device__ __forceinline__ void store_strip(uint32_t row0, uint32_t c0, uint32_t c1, const uint32_t (&a)[4][4])
+// whether one of the four bf16 scales is 2048 or more in size (0x4500): adding 0x3b00 to such a half, its sign removed, sets its top bit
+__device__ __forceinline__ bool large_scale(const uint2 s) { return ((((s.x & 0x7fff7fffu) + 0x3b003b00u) | ((s.y & 0x7fff7fffu) + 0x3b003b00u)) & 0x80008000u) != 0u; }
+// the same for 32 columns of the int8 format (16 bytes per lane)
+__device__ __forceinline__ void convert_strip_i8(const uint4& w, uint32_t* r)
 {
-    sts128(row0 + c0, a[0][0], a[0][2], a[1][0], a[1][2]);
-    sts128(row0 + c1, a[2][0], a[2][2], a[3][0], a[3][2]);
-    sts128(row0 + 1024 + c0, a[0][1], a[0][3], a[1][1], a[1][3]);
-    sts128(row0 + 1024 + c1, a[2][1], a[2][3], a[3][1], a[3][3]);
+    dec_i8(w.x, r[0], r[2]); dec_i8(w.y, r[1], r[3]); dec_i8(w.z, r[4], r[6]); dec_i8(w.w, r[5], r[7]);
 }
 
 // bf16 pair (rows g, g + 8 of a strip) -> two fp16x2 broadcast registers
@@ -348,44 +381,81 @@ __device__ __forceinline__ void scale_pair(uint32_t bf2, uint32_t& s_lo, uint32_
     s_lo = *(const uint32_t*) &lo; s_hi = *(const uint32_t*) &hi;
 }
 
-template <int NMAT>
+// shared memory: the packed codes (four 64-row x 128-column blocks of 4 KB and their scales) and the inputs (two 64-column tiles) of
+// the stages in flight. Codes are requested NCODE stages ahead (84 KB per SM: more than the 45 KB that cover a microsecond at the
+// memory's full rate), inputs NB stages ahead; the converted weights never come here.
 struct PfSmem
 {
-    static constexpr int STAGES = NMAT == 2 ? 3 : 4;
-    static constexpr int A_BYTES = TM * TK * 2;             // 16 KB per matrix
-    static constexpr int B_BYTES = TN * TK * 2;             // 32 KB
-    static constexpr int STAGE = NMAT * A_BYTES + B_BYTES;
-    static constexpr int bars = STAGES * STAGE;             // full_a[S], full_b[S], empty[S], done[2], tmem_free[2]
-    static constexpr int misc = bars + (3 * STAGES + 4) * 8;
+    static constexpr int NCODE = 5, NB = 4;
+    static constexpr int CODE_SLOT = 4 * 4096 + 4 * 128;
+    static constexpr int B_TILE = TN * TK * 2, B_SLOT = 2 * B_TILE;
+    static constexpr int b = 0;
+    static constexpr int code = NB * B_SLOT;
+    static constexpr int bars = code + NCODE * CODE_SLOT;   // code_full, code_empty [NCODE], b_full, b_empty [NB], a_full, a_empty [2], done, acc_free [2]
+    static constexpr int misc = bars + (2 * NCODE + 2 * NB + 8) * 8;
     static constexpr int total = misc + 32 + 1024;          // + slack to align the base to 1024
 };
+// tensor memory: columns 0..255 accumulators (two slots of 128: a block of up to 64 picks takes one slot for its two accumulators, a larger
+// one both), columns 256..511 two stages of converted weights (two matrices x 128 columns of fp16 = 64 words each)
+constexpr int TMEM_COLS = 512, TMEM_A = 256;
 
-// NMAT = 2: gate and up over one input tile, SiLU epilogue. NMAT = 1: down, scatter-add epilogue.
-template <int NMAT>
-__global__ void __launch_bounds__(pf_threads(NMAT), 1) prefill_gemm_kernel(const __grid_constant__ CUtensorMap tmap, const GemmArgs a)
+// The accumulator slots of a block's successive tiles; every role steps through the same sequence.
+struct AccSeq
 {
-    using L = PfSmem<NMAT>;
+    uint32_t small = 0, u0 = 0, u1 = 0, d0 = 0, d1 = 0;      // next slot of a small tile; tiles so far that took slot 0 / 1, that completed on slot 0 / 1
+    uint32_t mask, slot, up;                 // this tile: slots taken (bits), first slot, column distance of the second accumulator
+    uint32_t need0, need1, done_par;         // earlier uses of each slot; parity of the tile's completion barrier
+    __device__ __forceinline__ void next(int n)
+    {
+        const bool big = n > 64;
+        slot = big ? 0u : small; mask = big ? 3u : 1u << small; up = big ? 128u : 64u;
+        if (!big) small ^= 1u;
+        need0 = u0; need1 = u1;
+        u0 += mask & 1u; u1 += mask >> 1;
+        done_par = (slot ? d1 : d0) & 1u;
+        d0 += slot ^ 1u; d1 += slot;
+    }
+};
+
+// One item: a sub-block of a row block's picks (<= TN, one expert) x one 128-channel tile of gate and of up, or two 128-channel tiles of down.
+struct ItemPos { int e, pos0, n, ct, nmat; };
+template <bool DOWN>
+__device__ __forceinline__ ItemPos item_pos(const GemmArgs& a, int item, int nct)
+{
+    ItemPos it;
+    const int rs = item / nct;
+    it.ct = item - rs * nct;
+    const int rb = a.nsub == 1 ? rs : rs / a.nsub, sub = a.nsub == 1 ? 0 : rs - rb * a.nsub;
+    const int4 r = __ldg((const int4*) a.rbt + rb);
+    it.e = r.x; it.pos0 = r.y + sub * TN; it.n = min(r.z - sub * TN, TN);
+    it.nmat = DOWN ? (2 * it.ct + 1 < a.N / TM ? 2 : 1) : 2;
+    return it;
+}
+
+// DOWN = false: gate and up over one input tile, SiLU read-out. DOWN = true: two channel tiles of down, scatter-add read-out.
+template <bool DOWN>
+__global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap16, const __grid_constant__ GemmArgs a)
+{
+    using L = PfSmem;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t sbase = (raw + 1023u) & ~1023u;
     unsigned char* smem = smem_raw + (sbase - raw);
-    const uint32_t full_a = sbase + L::bars, full_b = full_a + L::STAGES * 8, empty = full_b + L::STAGES * 8,
-                   done = empty + L::STAGES * 8, tmem_free = done + 2 * 8;      // done[NACC], tmem_free[NACC]
+    const uint32_t code_full = sbase + L::bars, code_empty = code_full + L::NCODE * 8, b_full = code_empty + L::NCODE * 8, b_empty = b_full + L::NB * 8,
+                   a_full = b_empty + L::NB * 8, a_empty = a_full + 16, done = a_empty + 16, acc_free = done + 16;
     uint32_t* tmem_slot = (uint32_t*) (smem + L::misc);
     volatile int* abort_flag = (volatile int*) (smem + L::misc + 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // Accumulators in tensor memory: gate + up fill all 512 columns; down needs 256 and keeps two sets, so the MMAs of the
-    // next tile run while this tile's sums are read out.
-        constexpr int TMEM_COLS = 512, NACC = NMAT == 2 ? 1 : 2;
 
     if (threadIdx.x == 0)
     {
-        for (int i = 0; i < L::STAGES; ++i) { mbar_init(full_a + i * 8, NMAT == 2 ? NDQ : NDQ / 2); mbar_init(full_b + i * 8, 1); mbar_init(empty + i * 8, 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(done + i * 8, 1); mbar_init(tmem_free + i * 8, nepi(NMAT)); }
+        for (int i = 0; i < L::NCODE; ++i) { mbar_init(code_full + i * 8, 1); mbar_init(code_empty + i * 8, NDQ / 2); }
+        for (int i = 0; i < L::NB; ++i) { mbar_init(b_full + i * 8, 1); mbar_init(b_empty + i * 8, 2); }
+        for (int i = 0; i < 2; ++i) { mbar_init(a_full + i * 8, NDQ / 2); mbar_init(a_empty + i * 8, 2); mbar_init(done + i * 8, 2); mbar_init(acc_free + i * 8, NEPI); }
         *abort_flag = 0;
         fence_barrier_init();
     }
-    if (warp == NDQ + 1)
+    if (warp == NDQ + 2)
     {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -395,197 +465,255 @@ __global__ void __launch_bounds__(pf_threads(NMAT), 1) prefill_gemm_kernel(const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    const int KB = a.K / 64, KBT = KB * a.kfold, NCT = a.N / TM;     // KB 64-column blocks of the weights, KBT ring stages per tile
+    const int KS = a.K / 128, KST = KS * a.kfold;                    // 128-column stages of the weights / of a tile
+    const int NCT = DOWN ? (a.N / TM + 1) / 2 : a.N / TM;
 #ifdef HMOE_PROBE_WAITS
     unsigned long long pacc_[16] = {};
 #endif
     PROBE_T0();
-    const int nitems = a.plan->nrb * NCT;
+    const int nitems = a.plan->nrb * a.nsub * NCT;
 
     if (warp < NDQ)
     {
-        // ---- dequantise: one 16-row strip of one 64-row unit per warp and stage. gate_up: 2 matrices x 2 units x 4 strips =
-        // 16 strip-blocks per stage, one per warp. down: 8 strip-blocks per stage; warps 0-7 take the even pairs of stages, warps
-        // 8-15 the odd ones (in pairs of stages, see below). The packed words are fetched two of the warp's steps ahead. These warps
-        // do nothing else: they stream from tile to tile and stop only when the ring is full, so the MMA thread always finds its
-        // next stages.
-        const int g = lane >> 2, q = lane & 3;
-        const int strip = warp & 3, unit = (warp >> 2) & 1, mat = NMAT == 2 ? warp >> 3 : 0;
-        const int kb0 = NMAT == 2 ? 0 : warp >> 3, kstep = NMAT == 2 ? 1 : 2;
-        // shared address of this lane's row g in slot 0, and its two 16-byte columns under the 128-byte swizzle
-        const uint32_t row_off = sbase + mat * L::A_BYTES + (unit * 8 + strip * 2) * 1024 + g * 128;
-        const uint32_t c0 = (uint32_t) (((2 * q) ^ g) << 4), c1 = (uint32_t) (((2 * q + 1) ^ g) << 4);
+        // ---- convert: two groups of eight warps take the stages in turn, so that one group's waits (for codes, for its operand slot, for its
+        // stores) lie under the other's arithmetic. Warp w of a group takes, of matrix w / 4, the 32 rows of tensor-memory lane
+        // quarter w % 4 (a warp can only reach the quarter that matches its number) as two 16-row strips. In down's last item of an
+        // odd number of channel tiles the second tile's warps convert whatever the slot holds; nothing reads it.
+        const int g = lane >> 2, quarter = warp & 3, mat = (warp >> 2) & 1;
+        const uint32_t group = warp >> 3;
+        const uint32_t code0 = sbase + L::code + (mat * 2 + (quarter >> 1)) * 4096 + (quarter & 1) * 1024 + lane * 16;
+        const uint32_t sc0 = sbase + L::code + 4 * 4096 + (mat * 2 + (quarter >> 1)) * 128 + (g * 8 + (quarter & 1) * 4) * 2;
+        const uint32_t ta = tmem + TMEM_A + group * 128 + mat * 64 + ((uint32_t) (quarter * 32) << 16);      // the group's operand slot
+        uint32_t sc = 0, cph = 0, sb = 0, bph = 0, turn = 0, aph = 0;          // code ring, input ring; whose stage it is; parity of the operand slot
         bool ok = true;
-        uint32_t tile_n = 0;
-        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, ++tile_n)
+        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x)
         {
-            if (*abort_flag) { ok = false; break; }
-            const int rb = item / NCT, ct = item % NCT, e = a.rbt[4 * rb];
-            const void* wp = e < a.n_local ? (const void*) (mat ? a.w1[e] : a.w0[e]) : (mat ? a.sh_w1 : a.sh_w0);
-            const void* sp = e < a.n_local ? (const void*) (mat ? a.s1[e] : a.s0[e]) : (mat ? a.sh_s1 : a.sh_s0);
-            if (a.sh_i8 && e >= a.n_local)
-            {
-                // The shared expert in the reference's int8 format (runtime/tier/tier_split.py:495-514): 2 KB units of 64 rows x 32
-                // columns, 16 bytes per lane and strip = the fragments of two 16-column steps; a stage takes two units. One ninth
-                // of the work at most, so no prefetch queue: the two loads of a stage are issued, converted and stored in turn.
-                // Its fp32 row scales are applied by the read-out.
-                const char* w8 = (const char*) wp + ((size_t) (2 * ct + unit) * (a.K / 32) * 4 + strip) * 512 + lane * 16;
-                const uint32_t it0 = tile_n * (uint32_t) KBT;
-                for (int kb = kb0; kb < KBT && ok; kb += kstep)
-                {
-                    const int kbw = kb >= KB ? kb - KB : kb;
-                    const uint4 wa = ldg128_nc(w8 + (size_t) (2 * kbw) * 2048), wb = ldg128_nc(w8 + (size_t) (2 * kbw + 1) * 2048);
-                    uint32_t cv[4][4];
-                    dec_i8(wa.x, cv[0][0], cv[0][1]); dec_i8(wa.y, cv[0][2], cv[0][3]); dec_i8(wa.z, cv[1][0], cv[1][1]); dec_i8(wa.w, cv[1][2], cv[1][3]);
-                    dec_i8(wb.x, cv[2][0], cv[2][1]); dec_i8(wb.y, cv[2][2], cv[2][3]); dec_i8(wb.z, cv[3][0], cv[3][1]); dec_i8(wb.w, cv[3][2], cv[3][3]);
-                    const uint32_t gi = it0 + kb, s = gi % L::STAGES;
-                    if (gi >= (uint32_t) L::STAGES && !mbar_wait(empty + s * 8, ((gi / L::STAGES) - 1) & 1, abort_flag, a.status)) { ok = false; break; }
-                    store_strip(row_off + s * L::STAGE, c0, c1, cv);
-                    fence_proxy_async();
-                    __syncwarp();
-                    mbar_arrive_if(full_a + s * 8, lane == 0);
-                }
-                continue;
-            }
-            // One step of a warp = one 128-column scale group = two consecutive ring stages: two 16-byte code words and one scale
-            // word per lane. gate_up: every warp takes every pair of stages; down: warps 0-7 the even pairs, warps 8-15 the odd ones.
-            const int NPW = KB >> 1, NP = KBT >> 1;                  // pairs in one pass over the weights / in the tile
-            const int j0 = NMAT == 2 ? 0 : warp >> 3;
-            constexpr int JSTEP = NMAT == 2 ? 1 : 2;
-            const char* wbase = (const char*) wp + ((size_t) (2 * ct + unit) * KB * 4 + strip) * 512 + lane * 16;
-            const char* sbase_p = (const char*) sp + ((size_t) (2 * ct + unit) * (a.K / 128) * 64 + g * 8 + 2 * strip) * 2;
-            // the warp's ring slot and the parity of the slot's current use, stepped from stage to stage (no division per stage)
-            const uint32_t gi0 = tile_n * (uint32_t) KBT + 2 * j0;
-            uint32_t s = gi0 % L::STAGES, ph = (gi0 / L::STAGES) & 1;
+            const ItemPos it = item_pos<DOWN>(a, item, NCT);
+            if (it.n <= 0) continue;
+            if (*abort_flag) break;
+            const bool i8 = a.sh_i8 && it.e >= a.n_local;
+            auto code_wait = [&]() -> bool { PROBE_T0(); const bool w_ = mbar_wait(code_full + sc * 8, cph, abort_flag, a.status); if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(10); return w_; };
+            auto code_step = [&]() { if (++sc == (uint32_t) L::NCODE) { sc = 0; cph ^= 1; } };
+            auto code_release = [&]() {
+                __syncwarp();
+                mbar_arrive_if(code_empty + sc * 8, lane == 0);
+                code_step();
+            };
+            auto slot_wait = [&]() -> bool {
+                PROBE_T0(); const bool w_ = mbar_wait(a_empty + group * 8, aph ^ 1, abort_flag, a.status); if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(4);
+                tc_fence_after();
+                return w_;
+            };
+            // both strips are stored: hand the slot to the MMA warps. One warp also makes sure that the stage's inputs are in, so that the
+            // MMA warps have one barrier to wait for.
+            auto put = [&]() -> bool {
+                PROBE_T0();
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
+                bool w_ = true;
+                if ((warp & 7) == 0) w_ = mbar_wait(b_full + sb * 8, bph, abort_flag, a.status);
+                __syncwarp();
+                mbar_arrive_if(a_full + group * 8, lane == 0);
+                if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(9);
+                aph ^= 1;
+                return w_;
+            };
             auto run = [&](auto grouped_tag) {
                 constexpr bool GROUPED = decltype(grouped_tag)::value;
-                // the code words and scale pairs of the warp's next two steps, in flight while the current step is converted
-                uint4 qa[2] = {}, qb[2] = {}; uint32_t qs[2] = {};
-                auto fetch = [&](int pj, uint4& wa, uint4& wb, uint32_t& sc) {
-                    if (pj >= NP) return;
-                    const int jw = pj >= NPW ? pj - NPW : pj;               // second pass over the weights for the lo halves
-                    const char* p = wbase + (size_t) jw * 4096;
-                    wa = ldg128_nc(p); wb = ldg128_nc(p + 2048);
-                    if (GROUPED) sc = __ldg((const uint32_t*) (sbase_p + (size_t) jw * 128));
-                };
-                // the converted strip into ring slot s (a fresh slot passes at once: its barrier's preceding phase counts as
-                // complete), the slot handed to the MMA thread, s stepped
-                auto put = [&](const uint32_t (&cv)[4][4]) -> bool {
-                    { PROBE_T0(); const bool w_ = mbar_wait(empty + s * 8, ph ^ 1, abort_flag, a.status); if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(4); if (PROBE_ON(threadIdx.x == 15 * 32)) PROBE_ADD(10); if (!w_) return false; }
-                    PROBE_T0();
-                    store_strip(row_off + s * L::STAGE, c0, c1, cv);
-                    fence_proxy_async();
-                    __syncwarp();
-                    mbar_arrive_if(full_a + s * 8, lane == 0);
-                    if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(9);
-                    if (++s == (uint32_t) L::STAGES) { s = 0; ph ^= 1; }
-                    return true;
-                };
-                fetch(j0, qa[0], qb[0], qs[0]);
-                fetch(j0 + JSTEP, qa[1], qb[1], qs[1]);
-                uint32_t cv[4][4], s_lo = 0, s_hi = 0;                      // the converted strip of the warp's next stage
-                if (GROUPED) scale_pair(qs[0], s_lo, s_hi);
-                convert_strip(qa[0], s_lo, s_hi, GROUPED, cv);
-                for (int j = j0; j < NP && ok; j += 2 * JSTEP)
+                for (int j = 0; j < KST; ++j, turn ^= 1)
                 {
-                    #pragma unroll
-                    for (int u = 0; u < 2; ++u)
+                    if (turn != group) code_step();
+                    else
                     {
-                        const int jj = j + u * JSTEP;
-                        if (jj >= NP) break;
-                        if (!put(cv)) { ok = false; break; }
-                        convert_strip(qb[u], s_lo, s_hi, GROUPED, cv);      // before the wait for the second slot
-                        if (!put(cv)) { ok = false; break; }
-                        if (JSTEP == 2) { s += 2; if (s >= (uint32_t) L::STAGES) { s -= L::STAGES; ph ^= 1; } }     // the other warps' pair
-                        fetch(jj + 2 * JSTEP, qa[u], qb[u], qs[u]);
-                        if (GROUPED) scale_pair(qs[u ^ 1], s_lo, s_hi);     // the next pair's first stage, converted before its slot is waited for
-                        convert_strip(qa[u ^ 1], s_lo, s_hi, GROUPED, cv);
+                        if (!code_wait()) { ok = false; return; }
+                        const uint32_t at = code0 + sc * L::CODE_SLOT;
+                        uint2 sp = make_uint2(0, 0);
+                        if (GROUPED) sp = lds64(sc0 + sc * L::CODE_SLOT);
+                        auto strips = [&](auto mode_tag) {
+                            constexpr Conv MODE = decltype(mode_tag)::value;
+                            uint32_t r[32], s_lo = 0, s_hi = 0;
+                            uint4 wa = lds128(at), wb = lds128(at + 2048);
+                            if (GROUPED) scale_pair(sp.x, s_lo, s_hi);
+                            convert_strip<MODE>(wa, s_lo, s_hi, r);
+                            convert_strip<MODE>(wb, s_lo, s_hi, r + 16);
+                            wa = lds128(at + 512); wb = lds128(at + 2048 + 512);
+                            if (!slot_wait()) { ok = false; return; }
+                            tmem_st_16x256(ta, r);
+                            if (GROUPED) scale_pair(sp.y, s_lo, s_hi);
+                            convert_strip<MODE>(wa, s_lo, s_hi, r);
+                            convert_strip<MODE>(wb, s_lo, s_hi, r + 16);
+                            code_release();
+                            tmem_st_16x256(ta + (16u << 16), r);
+                        };
+                        if (!GROUPED) strips(std::integral_constant<Conv, UNSCALED>());
+                        else if (__any_sync(0xffffffffu, large_scale(sp))) strips(std::integral_constant<Conv, SCALED>());
+                        else strips(std::integral_constant<Conv, FUSED>());
+                        if (!ok || !put()) { ok = false; return; }
                     }
+                    if (++sb == (uint32_t) L::NB) { sb = 0; bph ^= 1; }
                 }
             };
-            if (a.grouped) run(std::true_type()); else run(std::false_type());
+            if (i8)
+            {
+                // The shared expert in the reference's int8 format (runtime/tier/tier_split.py:495-514): 2 KB units of 64 rows x 32
+                // columns, so a code slot holds 64 columns and a stage takes two. Its fp32 row scales are applied by the read-out.
+                for (int j = 0; j < KST && ok; ++j, turn ^= 1)
+                {
+                    if (turn != group) { code_step(); code_step(); }
+                    else
+                    {
+                        if (!slot_wait()) { ok = false; break; }
+                        for (int h = 0; h < 2 && ok; ++h)
+                        {
+                            if (!code_wait()) { ok = false; break; }
+                            const uint32_t at = code0 + sc * L::CODE_SLOT;
+                            uint32_t r[16];
+                            convert_strip_i8(lds128(at), r);
+                            convert_strip_i8(lds128(at + 2048), r + 8);
+                            tmem_st_16x256_half(ta + h * 32, r);
+                            convert_strip_i8(lds128(at + 512), r);
+                            convert_strip_i8(lds128(at + 2048 + 512), r + 8);
+                            tmem_st_16x256_half(ta + h * 32 + (16u << 16), r);
+                            code_release();
+                        }
+                        if (ok && !put()) ok = false;
+                    }
+                    if (++sb == (uint32_t) L::NB) { sb = 0; bph ^= 1; }
+                }
+            }
+            else if (a.grouped) run(std::true_type());
+            else run(std::false_type());
         }
     }
     else if (warp == NDQ)
     {
-        if (lane == 0)
+        // ---- codes: per stage (int8: half stage) one bulk copy of 4 KB per matrix and 64-row group, lanes 0..3, and its 128 bytes of scales, lanes 4..7
+        uint32_t s = 0, ph = 0;
+        bool ok = true;
+        const int blk = lane & 3, mat = blk >> 1, unit = blk & 1;
+        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x)
         {
-            uint32_t tile_n = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, ++tile_n)
-            {
-                const int pos0 = a.rbt[4 * (item / NCT) + 1], n = a.rbt[4 * (item / NCT) + 2];
-                // boxes of 64 rows: a row block with few picks brings in only the rows the MMA reads (n rounded up to 16 <= 64 nb)
-                const int nb = (n + 63) >> 6;
-                for (int kb = 0; kb < KBT; ++kb)
+            const ItemPos it = item_pos<DOWN>(a, item, NCT);
+            if (it.n <= 0) continue;
+            const bool sh = it.e >= a.n_local, i8 = a.sh_i8 && sh, scaled = a.grouped && !i8;
+            const bool second = !DOWN && mat;
+            const char* wp = (const char*) (sh ? (second ? a.sh_w1 : a.sh_w0) : (const void*) (second ? a.w1 : a.w0)[it.e]);
+            const char* sp = (const char*) (sh ? (second ? a.sh_s1 : a.sh_s0) : (const void*) (second ? a.s1 : a.s0)[it.e]);
+            const int gr = DOWN ? (2 * it.ct + mat) * 2 + unit : 2 * it.ct + unit;          // 64-row group
+            const char* src = lane < 4 ? wp + (size_t) gr * (a.K / 64) * (i8 ? 4096 : 2048) : sp + (size_t) gr * KS * 128;
+            const bool on = mat < it.nmat && (lane < 4 || (lane < 8 && scaled));
+            const uint32_t bytes = lane < 4 ? 4096 : 128, dst0 = sbase + L::code + (lane < 4 ? blk * 4096 : 4 * 4096 + blk * 128);
+            const uint32_t total = (uint32_t) it.nmat * 2 * (4096 + (scaled ? 128 : 0));
+            const int steps = i8 ? 2 * KS : KS;                      // copies of one pass over the weights
+            for (int f = 0; f < a.kfold && ok; ++f)
+                for (int j = 0; j < steps; ++j)
                 {
-                    const uint32_t it = tile_n * (uint32_t) KBT + kb, s = it % L::STAGES;
-                    { PROBE_T0(); const bool w_ = it < (uint32_t) L::STAGES || mbar_wait(empty + s * 8, ((it / L::STAGES) - 1) & 1, abort_flag, a.status); PROBE_ADD(6); if (!w_) { ok = false; break; } }
-                    mbar_expect_tx(full_b + s * 8, (uint32_t) nb * (TB * TK * 2));
-                    for (int b = 0; b < nb; ++b)
-                        tma_load_2d(sbase + s * L::STAGE + NMAT * L::A_BYTES + b * (TB * TK * 2), &tmap, kb * 64, pos0 + b * TB, full_b + s * 8);
+                    if (!mbar_wait(code_empty + s * 8, ph ^ 1, abort_flag, a.status)) { ok = false; break; }
+                    if (lane == 0) mbar_expect_tx(code_full + s * 8, total);
+                    __syncwarp();
+                    if (on) bulk_g2s(dst0 + s * L::CODE_SLOT, src + (size_t) j * bytes, bytes, code_full + s * 8);
+                    if (++s == (uint32_t) L::NCODE) { s = 0; ph ^= 1; }
                 }
-            }
         }
     }
     else if (warp == NDQ + 1)
     {
-        if (lane == 0)
+        // ---- inputs: the picks' 128 columns of a stage as two tiles of 64 columns, in boxes of 64 rows and, for the last rows, of 16, so that a
+        // block with few picks brings in little more than the rows the MMAs read (n rounded up to 16)
+        uint32_t s = 0, ph = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x)
         {
-            uint32_t tile_n = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, ++tile_n)
+            const ItemPos it = item_pos<DOWN>(a, item, NCT);
+            if (it.n <= 0) continue;
+            const int n16 = (it.n + 15) & ~15, nbig = n16 >> 6, nbox = nbig + ((n16 & 63) >> 4);
+            const int tile = lane / nbox, box = lane - tile * nbox, row = box < nbig ? box * 64 : nbig * 64 + (box - nbig) * 16;
+            const bool on = lane < 2 * nbox;
+            for (int j = 0; j < KST; ++j)
             {
-                const int n = a.rbt[4 * (item / NCT) + 2];
-                const uint32_t n16 = (uint32_t) ((n + 15) & ~15);
-                const uint32_t idesc = (1u << 4) | ((n16 >> 3) << 17) | ((uint32_t) (TM >> 4) << 24);
-                const uint32_t acc = tile_n % NACC, tacc = tmem + acc * 256;
-                // the accumulator set is free once the tile that used it last has been read out
-                { PROBE_T0(); const bool w_ = tile_n < (uint32_t) NACC || mbar_wait(tmem_free + acc * 8, ((tile_n / NACC) - 1) & 1, abort_flag, a.status); PROBE_ADD(2); if (!w_) break; }
+                { PROBE_T0(); const bool w_ = mbar_wait(b_empty + s * 8, ph ^ 1, abort_flag, a.status); if (PROBE_ON(lane == 0)) PROBE_ADD(6); if (!w_) { ok = false; break; } }
+                if (lane == 0) mbar_expect_tx(b_full + s * 8, (uint32_t) n16 * (2 * TK * 2));
+                __syncwarp();
+                if (on) tma_load_2d(sbase + L::b + s * L::B_SLOT + tile * L::B_TILE + row * (TK * 2), box < nbig ? &tmap : &tmap16, j * 128 + tile * 64, it.pos0 + row, b_full + s * 8);
+                if (++s == (uint32_t) L::NB) { s = 0; ph ^= 1; }
+            }
+        }
+    }
+    else if (warp < NDQ + 4)
+    {
+        // ---- MMA: one warp per accumulator (gate / up, or the two channel tiles); the whole warp steps through the stages, one elected lane
+        // issues. Between two stages' MMAs lie a few hundred cycles of waiting, fencing and committing while the converting warps take most of
+        // the issue slots (measured with one warp for both accumulators: 450 cycles per stage against 16 x 17 for the MMAs of a block of
+        // few picks); with two warps one's stage is under way meanwhile. All 512 columns are allocated, so the allocation starts at
+        // column 0 (checked here): the addresses of the operands are plain arithmetic on loop counters.
+        const uint32_t acc = warp - (NDQ + 2);
+        uint32_t sb = 0, sa = 0, aph = 0;
+        const uint64_t bdesc0 = smem_desc_sw128(sbase + L::b);
+        AccSeq seq;
+        bool ok = tmem == 0u;
+        if (!ok && lane == 0) { *abort_flag = 1; atomicOr(a.status, ST_WAIT_TIMEOUT); }
+        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x)
+        {
+            const ItemPos it = item_pos<DOWN>(a, item, NCT);
+            if (it.n <= 0) continue;
+            const uint32_t n16 = (uint32_t) ((it.n + 15) & ~15);
+            const uint32_t idesc = (1u << 4) | ((n16 >> 3) << 17) | ((uint32_t) (TM >> 4) << 24);
+            seq.next(it.n);
+            // the accumulators are free once the tiles that used their slots last have been read out
+            PROBE_T0();
+            if ((seq.mask & 1) && seq.need0 && !mbar_wait(acc_free, (seq.need0 - 1) & 1, abort_flag, a.status)) ok = false;
+            if ((seq.mask & 2) && seq.need1 && !mbar_wait(acc_free + 8, (seq.need1 - 1) & 1, abort_flag, a.status)) ok = false;
+            if (PROBE_ON(acc == 0)) PROBE_ADD(2);
+            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t d = seq.slot * 128 + acc * seq.up;
+            const bool live = !DOWN || (int) acc < it.nmat;
+            for (int j = 0; j < KST; ++j)
+            {
+                bool w;
+                { PROBE_T0(); w = mbar_wait(a_full + sa * 8, aph, abort_flag, a.status); if (PROBE_ON(acc == 0)) PROBE_ADD(0); }
+                if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
                 tc_fence_after();
-                for (int kb = 0; kb < KBT && ok; ++kb)
+                const uint32_t at = TMEM_A + sa * 128 + acc * 64;
+                const uint64_t bd = bdesc0 + sb * (L::B_SLOT >> 4);
+                if (elect_one())
                 {
-                    const uint32_t it = tile_n * (uint32_t) KBT + kb, s = it % L::STAGES, ph = (it / L::STAGES) & 1;
-                    { PROBE_T0(); const bool w_ = mbar_wait(full_a + s * 8, ph, abort_flag, a.status); PROBE_ADD(0); if (!w_) { ok = false; break; } }
-                    { PROBE_T0(); const bool w_ = mbar_wait(full_b + s * 8, ph, abort_flag, a.status); PROBE_ADD(1); if (!w_) { ok = false; break; } }
-                    tc_fence_after();
-                    const uint32_t at = sbase + s * L::STAGE, bt = at + NMAT * L::A_BYTES;
-                    #pragma unroll
-                    for (int k = 0; k < 4; ++k)
+                    if (live)
                     {
-                        const uint64_t bd = smem_desc_sw128(bt + k * 32);
-                        mma_f16_ss(tacc, smem_desc_sw128(at + k * 32), bd, idesc, (kb | k) != 0);
-                        if (NMAT == 2) mma_f16_ss(tacc + 256, smem_desc_sw128(at + L::A_BYTES + k * 32), bd, idesc, (kb | k) != 0);
+                        if (j == 0) mma_f16_ts<true>(d, at, bd, idesc); else mma_f16_ts<false>(d, at, bd, idesc);
+                        #pragma unroll
+                        for (int k = 1; k < 8; ++k) mma_f16_ts<false>(d, at + k * 8, bd + (k >> 2) * (L::B_TILE >> 4) + (k & 3) * 2, idesc);
                     }
-                    tc_commit(empty + s * 8);
+                    tc_commit(a_empty + sa * 8);
+                    tc_commit(b_empty + sb * 8);
+                    if (j + 1 == KST) tc_commit(done + seq.slot * 8);
                 }
-                if (ok) tc_commit(done + acc * 8);
+                __syncwarp();
+                if (++sa == 2) { sa = 0; aph ^= 1; }
+                if (++sb == (uint32_t) L::NB) sb = 0;
             }
         }
     }
     else
     {
-        // ---- read-out: warp NDQ + 2 + i reads the tensor-memory lanes of quarter (warp % 4) (a warp may only touch the quarter
-        // that matches its number), i.e. 32 output channels, for all picks of the tile, 16 columns at a time. gate_up: SiLU(gate)
-        // * up * routing weight -> fp16 activations; down: out[token] += scale * sum, one fp32 reduction per element (32 lanes =
-        // 32 consecutive channels = 128 contiguous bytes). Because these warps do nothing else, the read-out of a tile overlaps
-        // the dequantisation and (down: second accumulator set) the MMAs of the next one.
-        const int lq = warp & 3, chalf = (warp - (NDQ + 2)) >> 2;        // lane quarter; gate_up: which half of the columns
-        uint32_t tile_n = 0;
+        // ---- read-out: warp i reads the tensor-memory lanes of quarter i % 4, i.e. 32 output channels per accumulator. gate_up: SiLU(gate)
+        // * up * routing weight -> fp16 activations, the two warps of a quarter take half of the picks each; down: out[token] += scale *
+        // sum, one fp32 reduction per element (32 lanes = 32 consecutive channels = 128 contiguous bytes), one of the two channel
+        // tiles per warp. These warps do nothing else, so the read-out of a tile overlaps the conversion (and for blocks of up to 64 picks,
+        // which leave the other accumulator slot free, the MMAs) of the next one.
+        const int lq = warp & 3, half = (warp - (NDQ + 4)) >> 2;
+        AccSeq seq;
         bool ok = true;
-        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x, ++tile_n)
+        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x)
         {
+            const ItemPos it = item_pos<DOWN>(a, item, NCT);
+            if (it.n <= 0) continue;
             if (*abort_flag) break;
-            const int rb = item / NCT, ct = item % NCT;
-            const int e = a.rbt[4 * rb], pos0 = a.rbt[4 * rb + 1], n = a.rbt[4 * rb + 2];
-            (void) chalf;
-            const uint32_t acc = (uint32_t) (tile_n % NACC);
-            const uint32_t n16 = (uint32_t) ((n + 15) & ~15);
-            const int ch = ct * TM + lq * 32 + lane;
-            const int chp = (ch & ~63) + operand_pos(ch & 63);       // where the down GEMM expects this channel of the activations
-            const uint32_t tacc = tmem + acc * 256 + ((uint32_t) (lq * 32) << 16);
-            const int csplit = NMAT == 2 ? (((int) n16 + 31) >> 5) << 4 : (int) n16;      // gate_up: columns [0, csplit) and [csplit, n16)
-            const int cbeg = chalf ? csplit : 0, cend = chalf ? (int) n16 : csplit;
+            const int e = it.e, pos0 = it.pos0, n = it.n, n16 = (n + 15) & ~15;
+            seq.next(n);
+            const bool live = !DOWN || half < it.nmat;
+            const int ch = (DOWN ? 2 * it.ct + (live ? half : 0) : it.ct) * TM + lq * 32 + lane;
+            const uint32_t tacc = tmem + seq.slot * 128 + ((uint32_t) (lq * 32) << 16);
             // Everything the read-out needs besides the sums is fetched BEFORE the wait for the tile's last MMA, so that no global
             // load stands between that MMA and the release of the accumulators: the row scales, and in gate_up the
             // routing weights of the warp's columns (lane l holds picks cbeg + 32 i + l).
@@ -594,41 +722,40 @@ __global__ void __launch_bounds__(pf_threads(NMAT), 1) prefill_gemm_kernel(const
             {
                 const void* s0p = e < a.n_local ? (const void*) a.s0[e] : a.sh_s0;
                 sc0 = __ldg((const float*) s0p + ch);
-                if (NMAT == 2) { const void* s1p = e < a.n_local ? (const void*) a.s1[e] : a.sh_s1; sc1 = __ldg((const float*) s1p + ch); }
+                if (!DOWN) { const void* s1p = e < a.n_local ? (const void*) a.s1[e] : a.sh_s1; sc1 = __ldg((const float*) s1p + ch); }
             }
-            float wv[4] = {0.f, 0.f, 0.f, 0.f};
-            if constexpr (NMAT == 2)
+            if constexpr (!DOWN)
             {
+                const int csplit = ((n16 + 31) >> 5) << 4;          // the quarter's two warps take columns [0, csplit) and [csplit, n16)
+                const int cbeg = half ? csplit : 0, cend = half ? n16 : csplit;
+                float wv[2] = {0.f, 0.f};
                 #pragma unroll
-                for (int i = 0; i < 4; ++i) { const int pj = cbeg + 32 * i + lane; if (pj < n) wv[i] = __ldg(a.wt + pos0 + pj); }
-            }
-            { PROBE_T0(); const bool w_ = mbar_wait(done + acc * 8, (tile_n / NACC) & 1, abort_flag, a.status); if (PROBE_ON(threadIdx.x == (NDQ + 2) * 32)) PROBE_ADD(7); if (!w_) break; }
-            PROBE_T0();
-            tc_fence_after();
-            if constexpr (NMAT == 2)
-            {
-                // Eight columns at a time, one register set: with 72 registers per thread a second set in flight (the next eight columns'
-                // tensor-memory loads under the current eight's arithmetic) left the compiler too few registers to run the eight columns'
-                // exp / reciprocal / product chains side by side, and the read-out took twice as long (measured: 127 M against 62 M
-                // cycles per step over all SMs; the loads alone are 17 M). The tensor core waits for this read-out.
-                // The loops carry no branch per column: a conditional region per column costs convergence-barrier instructions that
-                // run one after the other (measured: ~70 cycles per column); the arithmetic runs for the padding columns too and
-                // only the store is predicated; the int8 mode is a compile-time variant of the whole loop.
-                uint32_t g0[8], u0[8];
+                for (int i = 0; i < 2; ++i) { const int pj = cbeg + 32 * i + lane; if (pj < n) wv[i] = __ldg(a.wt + pos0 + pj); }
+                { PROBE_T0(); const bool w_ = mbar_wait(done + seq.slot * 8, seq.done_par, abort_flag, a.status); if (PROBE_ON(threadIdx.x == (NDQ + 4) * 32)) PROBE_ADD(7); if (!w_) break; }
+                PROBE_T0();
+                tc_fence_after();
+                const int chp = (ch & ~63) + operand_pos(ch & 63);       // where the down GEMM expects this channel of the activations
+                // Eight columns at a time. The loops carry no branch per column: a conditional region per column costs
+                // convergence-barrier instructions that run one after the other (measured: ~70 cycles per column); the arithmetic runs
+                // for the padding columns too and only the store is predicated; the int8 mode is a compile-time variant of the whole loop.
                 auto read_out = [&](auto aq_tag) {
                     constexpr bool AQ = decltype(aq_tag)::value;
-                    auto emit = [&](const uint32_t (&gr)[8], const uint32_t (&ur)[8], int c0) {
-                        const int rel = c0 - cbeg, wi = rel >> 5, lb = rel & 31;
-                        const float wsel = wi == 0 ? wv[0] : wi == 1 ? wv[1] : wi == 2 ? wv[2] : wv[3];
+                    uint32_t g0[8], u0[8];
+                    for (int c0 = cbeg; c0 < cend; c0 += 8)
+                    {
+                        tmem_ld8(tacc + c0, g0); tmem_ld8(tacc + seq.up + c0, u0);
+                        tmem_ld_wait();
+                        const int rel = c0 - cbeg;
+                        const float wsel = rel < 32 ? wv[0] : wv[1];
                         float ws[8];
                         #pragma unroll
-                        for (int j = 0; j < 8; ++j) ws[j] = __shfl_sync(0xffffffffu, wsel, lb + j);
+                        for (int j = 0; j < 8; ++j) ws[j] = __shfl_sync(0xffffffffu, wsel, (rel & 31) + j);
                         #pragma unroll
                         for (int j = 0; j < 8; ++j)
                         {
                             const int p = c0 + j;
                             const float w = ws[j];
-                            const float gg = __uint_as_float(gr[j]) * sc0, uu = __uint_as_float(ur[j]) * sc1;
+                            const float gg = __uint_as_float(g0[j]) * sc0, uu = __uint_as_float(u0[j]) * sc1;
                             if (AQ)
                             {
                                 float v = gg / (1.f + expf(-gg)) * uu * w;
@@ -651,32 +778,31 @@ __global__ void __launch_bounds__(pf_threads(NMAT), 1) prefill_gemm_kernel(const
                                 if (p < n) a.act[(size_t) (pos0 + p) * a.N + chp] = v;
                             }
                         }
-                    };
-                    for (int c0 = cbeg; c0 < cend; c0 += 8)
-                    {
-                        tmem_ld8(tacc + c0, g0); tmem_ld8(tacc + 256 + c0, u0);
-                        tmem_ld_wait();
-                        emit(g0, u0, c0);
                     }
                 };
                 if (a.act_quant) read_out(std::true_type()); else read_out(std::false_type());
+                if (PROBE_ON(threadIdx.x == (NDQ + 4) * 32)) PROBE_ADD(8);
             }
             else
             {
-                // Sixteen columns at a time, two register sets in turn: the tensor-memory load of the next sixteen columns is in
-                // flight while the current sixteen go out as reductions. No branch per column here either: the padding columns
-                // add 0 to the row of the block's last pick.
-                uint32_t r0[16], r1[16];
+                { PROBE_T0(); const bool w_ = mbar_wait(done + seq.slot * 8, seq.done_par, abort_flag, a.status); if (PROBE_ON(threadIdx.x == (NDQ + 4) * 32)) PROBE_ADD(7); if (!w_) break; }
+                PROBE_T0();
+                tc_fence_after();
+                // Eight columns at a time. No branch per column here either: the padding columns add 0 to the row of the block's last pick.
+                const uint32_t td = tacc + half * seq.up;
                 auto read_out = [&](auto peer_tag) {
                     constexpr bool PEER = decltype(peer_tag)::value;
-                    auto emit = [&](const uint32_t (&r)[16], int c0, int tj) {
-                        int tks[16];
+                    for (int c0 = 0; c0 < n16; c0 += 8)
+                    {
+                        uint32_t r[8];
+                        tmem_ld8(td + c0, r);
+                        // lane j (and j + 8, ...) fetches the token of pick c0 + j while the tensor-memory load is in flight
+                        const int tj = __ldg(a.tok + pos0 + min(c0 + (lane & 7), n - 1));
+                        tmem_ld_wait();
                         #pragma unroll
-                        for (int j = 0; j < 16; ++j) tks[j] = __shfl_sync(0xffffffffu, tj, j);
-                        #pragma unroll
-                        for (int j = 0; j < 16; ++j)
+                        for (int j = 0; j < 8; ++j)
                         {
-                            const int tk = tks[j];
+                            const int tk = __shfl_sync(0xffffffffu, tj, j);
                             const float v = c0 + j < n ? __uint_as_float(r[j]) * sc0 : 0.f;
                             if (PEER)
                             {
@@ -687,40 +813,32 @@ __global__ void __launch_bounds__(pf_threads(NMAT), 1) prefill_gemm_kernel(const
                             }
                             else atomicAdd(a.out + (size_t) tk * a.N + ch, v);
                         }
-                    };
-                    // lane j (and j + 16) fetches the token of pick c0 + j while the tensor-memory load is in flight
-                    auto token_of = [&](int c0) { return __ldg(a.tok + pos0 + min(c0 + (lane & 15), n - 1)); };
-                    if (cbeg < cend) tmem_ld16(tacc + cbeg, r0);
-                    for (int c0 = cbeg; c0 < cend; c0 += 32)
-                    {
-                        const int ta = token_of(c0), tb = token_of(c0 + 16);
-                        tmem_ld_wait();
-                        if (c0 + 16 < cend) tmem_ld16(tacc + c0 + 16, r1);
-                        emit(r0, c0, ta);
-                        if (c0 + 16 < cend)
-                        {
-                            tmem_ld_wait();
-                            if (c0 + 32 < cend) tmem_ld16(tacc + c0 + 32, r0);
-                            emit(r1, c0 + 16, tb);
-                        }
                     }
                 };
-                if (a.rows_per_rank) read_out(std::true_type()); else read_out(std::false_type());
+                if (live) { if (a.rows_per_rank) read_out(std::true_type()); else read_out(std::false_type()); }
+                if (PROBE_ON(threadIdx.x == (NDQ + 4) * 32)) PROBE_ADD(8);
             }
             tc_fence_before();
             __syncwarp();
-            mbar_arrive_if(tmem_free + acc * 8, lane == 0);
-            if (PROBE_ON(threadIdx.x == (NDQ + 2) * 32)) PROBE_ADD(8);
+            #pragma unroll
+            for (int i = 0; i < 2; ++i) mbar_arrive_if(acc_free + i * 8, lane == 0 && (seq.mask >> i & 1));
         }
     }
 #ifdef HMOE_PROBE_WAITS
     if (threadIdx.x == 0) PROBE_ADD(15);
     #pragma unroll
-    for (int i = 0; i < 16; ++i) if (pacc_[i]) atomicAdd(&g_probe[(NMAT - 1) * 32 + i], pacc_[i]);
+    for (int i = 0; i < 16; ++i) if (pacc_[i] && !(warp >= NDQ + 2 && warp < NDQ + 4 && lane)) atomicAdd(&g_probe[(DOWN ? 0 : 1) * 32 + i], pacc_[i]);
 #endif
     tc_fence_before();
     __syncthreads();
-    if (warp == NDQ + 1)
+    if (*abort_flag && threadIdx.x == 0)
+    {
+        // a wait gave up: copies may still be in flight into this block's shared memory; leave them time to land
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 2000000ull) ;
+    }
+    __syncthreads();
+    if (warp == NDQ + 2)
     {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
@@ -741,14 +859,14 @@ encode_fn_t encode_fn()
     return f;
 }
 
-// row-major fp16 [rows][K] in boxes of 64 columns x 64 rows, 128-byte swizzle
-bool make_map(CUtensorMap* m, const void* ptr, int K, size_t rows)
+// row-major fp16 [rows][K] in boxes of 64 columns x `box_rows` rows, 128-byte swizzle
+bool make_map(CUtensorMap* m, const void* ptr, int K, size_t rows, int box_rows)
 {
     encode_fn_t f = encode_fn();
     if (!f) return false;
     cuuint64_t dims[2] = {(cuuint64_t) K, (cuuint64_t) rows};
     cuuint64_t strides[1] = {(cuuint64_t) K * 2};
-    cuuint32_t box[2] = {TK, TB}, es[2] = {1, 1};
+    cuuint32_t box[2] = {TK, (cuuint32_t) box_rows}, es[2] = {1, 1};
     return f(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*) ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -760,8 +878,8 @@ void set_gemm_attributes()
 {
     static DeviceOnce once;
     if (!once.first()) return;
-    cudaFuncSetAttribute(prefill_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, PfSmem<2>::total);
-    cudaFuncSetAttribute(prefill_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, PfSmem<1>::total);
+    cudaFuncSetAttribute(prefill_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PfSmem::total);
+    cudaFuncSetAttribute(prefill_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PfSmem::total);
 }
 
 struct WsLayout
@@ -845,20 +963,21 @@ int prefill_sorted_launch(const hmoe_layer* L, const void* x, int x_dtype, const
     __half* act = (__half*) (b + 512 + up256((size_t) npos * H * 2 * kf));
     set_plan_kernel<<<1, 1, 0, st>>>(plan, npos, nrb);
     gather_kernel<<<npos, 192, 0, st>>>(x, x_dtype == HMOE_BF16, tok, plan, H, act_quant, xg);
-    CUtensorMap mx, ma;
-    if (!make_map(&mx, xg, H * kf, (size_t) npos) || !make_map(&ma, act, I * kf, (size_t) npos)) return fail(HMOE_E_CUDA, "hmoe_prefill_sorted: cuTensorMapEncodeTiled failed");
+    CUtensorMap mx, ma, mx16, ma16;
+    if (!make_map(&mx, xg, H * kf, (size_t) npos, 64) || !make_map(&ma, act, I * kf, (size_t) npos, 64) || !make_map(&mx16, xg, H * kf, (size_t) npos, 16) ||
+        !make_map(&ma16, act, I * kf, (size_t) npos, 16)) return fail(HMOE_E_CUDA, "hmoe_prefill_sorted: cuTensorMapEncodeTiled failed");
     GemmArgs g;
-    g.grouped = L->group != 0; g.act_quant = act_quant; g.n_local = n_local; g.kfold = kf;
+    g.grouped = L->group != 0; g.act_quant = act_quant; g.n_local = n_local; g.kfold = kf; g.nsub = 2;                // the caller's row blocks hold up to 256 picks
     g.sh_i8 = L->shared_format == 1 && L->sh_gate_w != nullptr;
     g.plan = plan; g.rbt = rbt; g.tok = tok; g.wt = wt; g.act = act; g.out = out; g.status = status;
     g.rows_per_rank = 0;
     for (int p = 0; p < 8; ++p) g.out_peer[p] = nullptr;
     g.K = H; g.N = I; g.w0 = L->gate_w; g.w1 = L->up_w; g.s0 = L->gate_s; g.s1 = L->up_s;
     g.sh_w0 = L->sh_gate_w; g.sh_w1 = L->sh_up_w; g.sh_s0 = L->sh_gate_s; g.sh_s1 = L->sh_up_s;
-    prefill_gemm_kernel<2><<<sms, pf_threads(2), PfSmem<2>::total, st>>>(mx, g);
+    prefill_gemm_kernel<false><<<sms, PF_THREADS, PfSmem::total, st>>>(mx, mx16, g);
     g.K = I; g.N = H; g.w0 = L->down_w; g.w1 = nullptr; g.s0 = L->down_s; g.s1 = nullptr;
     g.sh_w0 = L->sh_down_w; g.sh_w1 = nullptr; g.sh_s0 = L->sh_down_s; g.sh_s1 = nullptr;
-    prefill_gemm_kernel<1><<<sms, pf_threads(1), PfSmem<1>::total, st>>>(ma, g);
+    prefill_gemm_kernel<true><<<sms, PF_THREADS, PfSmem::total, st>>>(ma, ma16, g);
     count_launches(4);
     const cudaError_t err = cudaGetLastError();
     return err == cudaSuccess ? HMOE_OK : fail(HMOE_E_CUDA, cudaGetErrorString(err));
@@ -921,20 +1040,21 @@ int prefill_launch(const hmoe_layer* L, const void* x, int x_dtype, const int64_
                          rbt, plan, st);
     if (rc) return rc;
     gather_kernel<<<w.rows_cap, 192, 0, st>>>(x, x_dtype == HMOE_BF16, tok, plan, H, act_quant, xg);
-    CUtensorMap mx, ma;
-    if (!make_map(&mx, xg, H * kf, (size_t) w.rows_cap) || !make_map(&ma, act, I * kf, (size_t) w.rows_cap)) return fail(HMOE_E_CUDA, "hmoe_prefill: cuTensorMapEncodeTiled failed");
+    CUtensorMap mx, ma, mx16, ma16;
+    if (!make_map(&mx, xg, H * kf, (size_t) w.rows_cap, 64) || !make_map(&ma, act, I * kf, (size_t) w.rows_cap, 64) ||
+        !make_map(&mx16, xg, H * kf, (size_t) w.rows_cap, 16) || !make_map(&ma16, act, I * kf, (size_t) w.rows_cap, 16)) return fail(HMOE_E_CUDA, "hmoe_prefill: cuTensorMapEncodeTiled failed");
     GemmArgs g;
-    g.grouped = L->group != 0; g.act_quant = act_quant; g.n_local = n_local; g.kfold = kf;
+    g.grouped = L->group != 0; g.act_quant = act_quant; g.n_local = n_local; g.kfold = kf; g.nsub = 1;
     g.sh_i8 = L->shared_format == 1 && L->sh_gate_w != nullptr;
     g.plan = plan; g.rbt = rbt; g.tok = tok; g.wt = wt; g.act = act; g.out = out; g.status = status;
     g.rows_per_rank = out_peer ? rows_per_rank : 0;
     for (int p = 0; p < 8; ++p) g.out_peer[p] = (out_peer && p < world) ? (float*) out_peer[p] : nullptr;
     g.K = H; g.N = I; g.w0 = L->gate_w; g.w1 = L->up_w; g.s0 = L->gate_s; g.s1 = L->up_s;
     g.sh_w0 = L->sh_gate_w; g.sh_w1 = L->sh_up_w; g.sh_s0 = L->sh_gate_s; g.sh_s1 = L->sh_up_s;
-    prefill_gemm_kernel<2><<<sms, pf_threads(2), PfSmem<2>::total, st>>>(mx, g);
+    prefill_gemm_kernel<false><<<sms, PF_THREADS, PfSmem::total, st>>>(mx, mx16, g);
     g.K = I; g.N = H; g.w0 = L->down_w; g.w1 = nullptr; g.s0 = L->down_s; g.s1 = nullptr;
     g.sh_w0 = L->sh_down_w; g.sh_w1 = nullptr; g.sh_s0 = L->sh_down_s; g.sh_s1 = nullptr;
-    prefill_gemm_kernel<1><<<sms, pf_threads(1), PfSmem<1>::total, st>>>(ma, g);
+    prefill_gemm_kernel<true><<<sms, PF_THREADS, PfSmem::total, st>>>(ma, ma16, g);
     count_launches(3);
     const cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return fail(HMOE_E_CUDA, cudaGetErrorString(err));
