@@ -4,7 +4,8 @@
 // sigmoid uses a fixed polynomial exp, so the selected experts are reproducible bit for bit by the CPU checker.
 //   logit[r][e]: lane L of a warp sums columns i*256 + L*8 + j (i outer, j inner) with fused multiply-adds, then five
 //   butterfly steps (xor 16, 8, 4, 2, 1) add the 32 partial sums.
-// One launch: the block that completes a group of four rows last also selects their experts. Router calls that overlap
+// Few rows, one launch: the block that completes a group of four rows last also selects their experts. Many rows: router_tile_kernel
+// for the logits, a second launch for the selections. Router calls that overlap
 // on one device take different counter sets in rotation (sixteen of them).
 #include <atomic>
 #include "hmoe_common.cuh"
@@ -439,19 +440,117 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
     if (r < R) topk_row(logits, bias, r, E, topk, scale, sel, rw, lane, false, scratch + warp * 512);
 }
 
+// Logits of many rows. What bounds them is the fp32 multiply-adds (the fixed order of the sums rules out the tensor cores), so the tile is
+// chosen for those: a lane keeps its share (columns i*256 + L*8 + j, as above) of 8 rows x 8 experts in 64 accumulators, so every value
+// that is read from shared memory and widened serves eight multiply-adds. (The kernel above serves four rows per weight and one expert per
+// input: shared memory bounds it, and every block stages its rows anew for eight experts.) Four warps = 16 rows x 16 experts per block, three
+// blocks per SM; the rows' and experts' 256-column pieces come in by asynchronous copies, LT_STAGES - 1 steps ahead. The 32 lanes' shares are
+// added by the butterfly's sums (xor 16, 8, 4, 2, 1), each step halving the values a lane still carries.
+// Measured, 8192 rows x 256 experts x 6144 columns: 2908 us with the kernel above, 668 us with this one (39 TFLOP/s); a variant with packed
+// fma.rn.f32x2 took 691 us, one fed by bulk copies of 512 bytes 849 us (one warp issuing 32 of them stalls its block).
+constexpr int LT_ROWS = 16, LT_EXP = 16, LT_STAGES = 4, LT_STAGE_BYTES = (LT_ROWS + LT_EXP) * 512;
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+template <bool BF>
+__device__ __forceinline__ float2 widen2(uint32_t w)
+{
+    if (BF) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    return __half22float2(*(const __half2*) &w);
+}
+
 template <bool XBF, bool WBF>
-void launch_logits(dim3 grid, size_t smem, cudaStream_t st, bool fused, const uint16_t* x, const uint16_t* wt, int R, int H, int E,
+__global__ void __launch_bounds__(128, 3) router_tile_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ wt, int R, int H, int E,
+                                                             float* __restrict__ logits)
+{
+    extern __shared__ __align__(128) unsigned char tsm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int e0 = blockIdx.x * LT_EXP, r0 = blockIdx.y * LT_ROWS, nr = R - r0 < LT_ROWS ? R - r0 : LT_ROWS, S = H / 256;
+    const uint32_t sbase = smem_u32(tsm);
+    // warp w brings rows w, w + 4, ... and experts likewise; rows beyond the last repeat it (their sums are not stored)
+    const uint16_t* xsrc[LT_ROWS / 4];
+    #pragma unroll
+    for (int k = 0; k < LT_ROWS / 4; ++k) { const int r = warp + 4 * k; xsrc[k] = x + (size_t) (r0 + (r < nr ? r : nr - 1)) * H + lane * 8; }
+    const uint16_t* wsrc = wt + (size_t) (e0 + warp) * H + lane * 8;
+    const uint32_t dst = sbase + warp * 512 + lane * 16;
+    uint32_t fill = 0;
+    auto request = [&](int i) {
+        if (i < S)
+        {
+            #pragma unroll
+            for (int k = 0; k < LT_ROWS / 4; ++k) { cp_async16(dst + fill + k * 2048, xsrc[k]); xsrc[k] += 256; }
+            #pragma unroll
+            for (int k = 0; k < LT_EXP / 4; ++k) cp_async16(dst + fill + LT_ROWS * 512 + k * 2048, wsrc + (size_t) (4 * k) * H);
+            wsrc += 256;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        fill = fill + LT_STAGE_BYTES == LT_STAGES * LT_STAGE_BYTES ? 0 : fill + LT_STAGE_BYTES;
+    };
+    #pragma unroll
+    for (int i = 0; i < LT_STAGES - 1; ++i) request(i);
+    float v[64];
+    #pragma unroll
+    for (int r = 0; r < 64; ++r) v[r] = 0.f;
+    uint32_t at = sbase + lane * 16;
+    const uint32_t xoff = (warp & 1) * 8 * 512, woff = (LT_ROWS + (warp >> 1) * 8) * 512;
+    #pragma unroll 1
+    for (int i = 0; i < S; ++i)
+    {
+        asm volatile("cp.async.wait_group %0;" ::"n"(LT_STAGES - 2) : "memory");
+        __syncthreads();                                      // step i is in, and everyone has read step i - 1, whose slot is refilled
+        request(i + LT_STAGES - 1);
+        uint4 xr[8], wr[8];
+        #pragma unroll
+        for (int k = 0; k < 8; ++k) { wr[k] = lds128(at + woff + k * 512); xr[k] = lds128(at + xoff + k * 512); }
+        at = at + LT_STAGE_BYTES >= sbase + LT_STAGES * LT_STAGE_BYTES ? at + LT_STAGE_BYTES - LT_STAGES * LT_STAGE_BYTES : at + LT_STAGE_BYTES;
+        #pragma unroll
+        for (int c = 0; c < 4; ++c)
+        {
+            auto word = [&](const uint4& v) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; };
+            float2 wf[8];
+            #pragma unroll
+            for (int p = 0; p < 8; ++p) wf[p] = widen2<WBF>(word(wr[p]));
+            #pragma unroll
+            for (int r = 0; r < 8; ++r)
+            {
+                const float2 f = widen2<XBF>(word(xr[r]));
+                #pragma unroll
+                for (int p = 0; p < 8; ++p) v[r * 8 + p] = __fmaf_rn(f.x, wf[p].x, v[r * 8 + p]);
+                #pragma unroll
+                for (int p = 0; p < 8; ++p) v[r * 8 + p] = __fmaf_rn(f.y, wf[p].y, v[r * 8 + p]);
+            }
+        }
+    }
+    // value index r * 8 + e: a lane with bit 4 / 3 / 2 / 1 / 0 set keeps the upper half of what is left
+    #pragma unroll
+    for (int o = 16, n = 32; o; o >>= 1, n >>= 1)
+    {
+        const bool hi = (lane & o) != 0;
+        #pragma unroll
+        for (int k = 0; k < n; ++k)
+        {
+            const float mine = hi ? v[k + n] : v[k], other = hi ? v[k] : v[k + n];
+            v[k] = __fadd_rn(mine, __shfl_xor_sync(0xffffffffu, other, o));
+        }
+    }
+    // lane l is left with values 2 l and 2 l + 1: row l / 4, experts 2 (l % 4) and + 1
+    const int r = (warp & 1) * 8 + (lane >> 2), e = e0 + (warp >> 1) * 8 + 2 * (lane & 3);
+    if (r < nr) *(float2*) (logits + (size_t) (r0 + r) * E + e) = make_float2(v[0], v[1]);
+}
+template <bool XBF, bool WBF>
+void launch_tile(cudaStream_t st, const uint16_t* x, const uint16_t* wt, int R, int H, int E, float* logits)
+{
+    static DeviceOnce once;
+    if (once.first()) cudaFuncSetAttribute(router_tile_kernel<XBF, WBF>, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_STAGES * LT_STAGE_BYTES);
+    router_tile_kernel<XBF, WBF><<<dim3(E / LT_EXP, (R + LT_ROWS - 1) / LT_ROWS), 128, LT_STAGES * LT_STAGE_BYTES, st>>>(x, wt, R, H, E, logits);
+}
+
+template <bool XBF, bool WBF>
+void launch_logits(dim3 grid, size_t smem, cudaStream_t st, const uint16_t* x, const uint16_t* wt, int R, int H, int E,
                    float* logits, const float* bias, int topk, float scale, int64_t* sel, __half* rw, int slot, unsigned* status)
 {
     static DeviceOnce once;
-    if (once.first())
-    {
-        cudaFuncSetAttribute(router_logits_kernel<XBF, WBF, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(router_logits_kernel<XBF, WBF, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    }
+    if (once.first()) cudaFuncSetAttribute(router_logits_kernel<XBF, WBF, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     const NormArgs na = {};
-    if (fused) router_logits_kernel<XBF, WBF, true, false><<<grid, RW * 32, smem, st>>>(x, wt, R, H, E, logits, bias, topk, scale, sel, rw, slot, na, status, PrepArgs(), DispArgs());
-    else router_logits_kernel<XBF, WBF, false, false><<<grid, RW * 32, smem, st>>>(x, wt, R, H, E, logits, bias, topk, scale, sel, rw, slot, na, status, PrepArgs(), DispArgs());
+    router_logits_kernel<XBF, WBF, true, false><<<grid, RW * 32, smem, st>>>(x, wt, R, H, E, logits, bias, topk, scale, sel, rw, slot, na, status, PrepArgs(), DispArgs());
 }
 
 template <bool WBF>
@@ -507,16 +606,32 @@ int router_launch(const void* x, int x_dtype, const void* wt, int w_dtype, const
     unsigned* status = (unsigned*) ws;
     float* logits = (float*) ((char*) ws + 256);
     const uint16_t* xp = (const uint16_t*) x; const uint16_t* wp = (const uint16_t*) wt;
-    // Up to CTR_GROUPS row groups the selection runs in the same launch (the last block of a row group does it); beyond,
-    // a second kernel selects.
-    const bool fused = (int) grid.y <= CTR_GROUPS;
-    const int slot = (int) (g_router_calls.fetch_add(1, std::memory_order_relaxed) % CTR_SLOTS);
+    // The tiled kernel costs about 4 us per 1024 columns however few the rows (25 us for 6144), the other one a wave of blocks per four rows x
+    // eight experts x resident blocks: measured, us, other / tiled, 6144 columns x 256 experts: 32 rows 23 / 25, 48 rows 29 / 25, 64 rows
+    // 37 / 25, 1024 rows 431 / 95; 2048 x 64 (three blocks per SM): 200 rows 14.5 / 16.9, 256 rows 20.3 / 16.9; 8192 x 32: 256 rows
+    // 27 / 29, 400 rows 39 / 29. So it takes over after two waves, or one where three or more blocks share an SM.
+    const int sms = device_sms();
+    if (sms <= 0) return fail(HMOE_E_CUDA, "hmoe_router: no current CUDA device");
+    const int per_sm = (int) (227u * 1024u / (smem + 1024)), waves = per_sm > 2 ? per_sm : 2;
+    const bool fused = (int) grid.y <= CTR_GROUPS && (long long) grid.x * grid.y <= (long long) waves * sms;
     const bool xb = x_dtype == HMOE_BF16, wb = w_dtype == HMOE_BF16;
-    if (!xb && !wb) launch_logits<false, false>(grid, smem, st, fused, xp, wp, R, H, E, logits, bias, topk, scale, sel, (__half*) rw, slot, status);
-    else if (!xb && wb) launch_logits<false, true>(grid, smem, st, fused, xp, wp, R, H, E, logits, bias, topk, scale, sel, (__half*) rw, slot, status);
-    else if (xb && !wb) launch_logits<true, false>(grid, smem, st, fused, xp, wp, R, H, E, logits, bias, topk, scale, sel, (__half*) rw, slot, status);
-    else launch_logits<true, true>(grid, smem, st, fused, xp, wp, R, H, E, logits, bias, topk, scale, sel, (__half*) rw, slot, status);
-    if (!fused) router_topk_kernel<<<(R + 7) / 8, 256, 0, st>>>(logits, bias, R, E, topk, scale, sel, (__half*) rw);
+    if (!fused)
+    {
+        if (!xb && !wb) launch_tile<false, false>(st, xp, wp, R, H, E, logits);
+        else if (!xb && wb) launch_tile<false, true>(st, xp, wp, R, H, E, logits);
+        else if (xb && !wb) launch_tile<true, false>(st, xp, wp, R, H, E, logits);
+        else launch_tile<true, true>(st, xp, wp, R, H, E, logits);
+        router_topk_kernel<<<(R + 7) / 8, 256, 0, st>>>(logits, bias, R, E, topk, scale, sel, (__half*) rw);
+    }
+    else
+    {
+        // the last block of a row group selects its experts in the same launch
+        const int slot = (int) (g_router_calls.fetch_add(1, std::memory_order_relaxed) % CTR_SLOTS);
+        if (!xb && !wb) launch_logits<false, false>(grid, smem, st, xp, wp, R, H, E, logits, bias, topk, scale, sel, (__half*) rw, slot, status);
+        else if (!xb && wb) launch_logits<false, true>(grid, smem, st, xp, wp, R, H, E, logits, bias, topk, scale, sel, (__half*) rw, slot, status);
+        else if (xb && !wb) launch_logits<true, false>(grid, smem, st, xp, wp, R, H, E, logits, bias, topk, scale, sel, (__half*) rw, slot, status);
+        else launch_logits<true, true>(grid, smem, st, xp, wp, R, H, E, logits, bias, topk, scale, sel, (__half*) rw, slot, status);
+    }
     count_launches(fused ? 1 : 2);
     const cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return fail(HMOE_E_CUDA, cudaGetErrorString(err));

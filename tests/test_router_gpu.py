@@ -34,6 +34,13 @@ def test_router_dtypes_bias_scale(oracle, xbf, wbf):
     _run(oracle, 3, 256, 32, 8, xbf, wbf, None, 1.0, seed=8)
 
 
+@pytest.mark.parametrize("R", [33, 50, 257, 401, 1025])
+@pytest.mark.parametrize("H,E,xbf,wbf", [(256, 32, 1, 1), (1280, 96, 0, 1), (2304, 256, 0, 0), (6400, 64, 1, 0)])
+def test_router_bit_exact_tiled_rows(oracle, R, H, E, xbf, wbf):
+    """Both sides of the tiled kernel's threshold, remainders of its 16-row tiles, fewer and more 256-column steps than its ring has stages."""
+    _run(oracle, R, H, E, 8, xbf, wbf, 0.05, 1.5, seed=R + H)
+
+
 def test_router_large_rows(oracle):
     _run(oracle, 1000, 512, 128, 8, 1, 1, 0.05, 1.0, seed=9)
 
