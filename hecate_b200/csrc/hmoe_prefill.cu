@@ -12,7 +12,7 @@
 // memory, the picks of one row block (<= 128, one expert) the N operand in shared memory, fp32 accumulators in tensor memory. An
 // item is a row block x two 128-channel tiles (gate and up, or two tiles of down) over the same inputs, so that every input tile
 // feeds two MMA sequences. Per 128-column stage (one scale group):
-//   warp 16    brings the packed codes and scales into shared memory by 1-D bulk copies, five stages ahead;
+//   warp 16    brings the packed codes and scales into shared memory by 1-D bulk copies, four stages ahead;
 //   warps 0-15 in two groups that take the stages in turn: 16 bytes of codes per lane and strip -> fp16 (times the bf16 group scale)
 //              -> tcgen05.st. The stored fragment order of the codes is the row / word order of the 16x256b store, so the weights never
 //              pass through shared memory as fp16: at N <= 128 reading a 128-row operand from shared memory for every MMA, and writing it
@@ -26,6 +26,11 @@
 // Measured (256 experts of 6144 x 2048, us per call before -> after, before: fp16 weights staged through shared memory, row blocks of up
 // to 256 picks): 777 rows, Zipf(1.1) 2872 -> 1735; 2048 rows, fp32 row scales 2753 -> 1821; 8192 rows, Zipf(1.1) 6821 -> 6416 (the last two at
 // 1.45 GHz under the power cap).
+// The converting warps' issue slots are what a stage of few picks waits for (measured alone, four warps on a scheduler: 280 cycles per 16 words
+// of group-scaled codes, 210 of plain ones; beside them eight MMAs of 16 picks take 1240 cycles to issue instead of 470), so all that is not
+// conversion is kept short: the stage's inputs count their bytes on the barrier that the MMA warps wait for, a group steps over the other
+// group's stages, and slots and parities follow from running numbers. moe.prefill on random picks, us before -> after: scale groups, 64 rows
+// 1075 -> 998, 256 rows 1296 -> 1210, 2048 rows 1850 -> 1775; row scales, 2048 rows 1808 -> 1627, 4096 rows 3170 -> 2900.
 // Blocks are persistent (one per SM) over (row block, channel tile) items, channel tile fastest, so the blocks working at
 // the same time share one input tile and one expert's weights through L2.
 // Every wait is bounded (see mbar_wait); tensor memory is released by the warp that allocated it on every path.
@@ -295,6 +300,22 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr)
     return v;
 }
 
+// Bounded wait like mbar_wait in fewer instructions (these kernels' converting warps leave few issue slots to spare). The first try is a short
+// one: parked for long from the first try on, the thread wakes up later (measured: 64 to 2048 rows 3 to 7 % slower).
+__device__ __forceinline__ bool pf_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned* status)
+{
+    if (mbar_try(bar, parity)) return true;
+    unsigned long long t0 = 0;
+    while (!mbar_try_hint(bar, parity, 20000u))
+    {
+        if (*abort_flag) return false;
+        const unsigned long long now = globaltimer_ns();
+        if (t0 == 0) t0 = now;
+        else if (now - t0 > 1000000000ull) { *abort_flag = 1; if (status) atomicOr(status, ST_WAIT_TIMEOUT); return false; }
+    }
+    return true;
+}
+
 struct GemmArgs
 {
     int K, N;                 // reduction length and output channels of the matrix (gate_up: K = H, N = I; down: K = I, N = H)
@@ -382,17 +403,17 @@ __device__ __forceinline__ void scale_pair(uint32_t bf2, uint32_t& s_lo, uint32_
 }
 
 // shared memory: the packed codes (four 64-row x 128-column blocks of 4 KB and their scales) and the inputs (two 64-column tiles) of
-// the stages in flight. Codes are requested NCODE stages ahead (84 KB per SM: more than the 45 KB that cover a microsecond at the
-// memory's full rate), inputs NB stages ahead; the converted weights never come here.
+// the stages in flight. Codes are requested NCODE stages ahead (68 KB per SM: more than the 45 KB that cover a microsecond at the
+// memory's full rate; five or seven slots measured no faster), inputs NB stages ahead; the converted weights never come here.
 struct PfSmem
 {
-    static constexpr int NCODE = 5, NB = 4;
+    static constexpr int NCODE = 4, NB = 4;                  // powers of two: a running stage number gives slot and parity
     static constexpr int CODE_SLOT = 4 * 4096 + 4 * 128;
     static constexpr int B_TILE = TN * TK * 2, B_SLOT = 2 * B_TILE;
     static constexpr int b = 0;
     static constexpr int code = NB * B_SLOT;
-    static constexpr int bars = code + NCODE * CODE_SLOT;   // code_full, code_empty [NCODE], b_full, b_empty [NB], a_full, a_empty [2], done, acc_free [2]
-    static constexpr int misc = bars + (2 * NCODE + 2 * NB + 8) * 8;
+    static constexpr int bars = code + NCODE * CODE_SLOT;   // code_full, code_empty [NCODE], b_empty, a_full [NB], a_empty, done, acc_free [2]
+    static constexpr int misc = bars + (2 * NCODE + 2 * NB + 6) * 8;
     static constexpr int total = misc + 32 + 1024;          // + slack to align the base to 1024
 };
 // tensor memory: columns 0..255 accumulators (two slots of 128: a block of up to 64 picks takes one slot for its two accumulators, a larger
@@ -441,8 +462,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t sbase = (raw + 1023u) & ~1023u;
     unsigned char* smem = smem_raw + (sbase - raw);
-    const uint32_t code_full = sbase + L::bars, code_empty = code_full + L::NCODE * 8, b_full = code_empty + L::NCODE * 8, b_empty = b_full + L::NB * 8,
-                   a_full = b_empty + L::NB * 8, a_empty = a_full + 16, done = a_empty + 16, acc_free = done + 16;
+    const uint32_t code_full = sbase + L::bars, code_empty = code_full + L::NCODE * 8, b_empty = code_empty + L::NCODE * 8, a_full = b_empty + L::NB * 8,
+                   a_empty = a_full + L::NB * 8, done = a_empty + 16, acc_free = done + 16;
     uint32_t* tmem_slot = (uint32_t*) (smem + L::misc);
     volatile int* abort_flag = (volatile int*) (smem + L::misc + 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -450,8 +471,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
     if (threadIdx.x == 0)
     {
         for (int i = 0; i < L::NCODE; ++i) { mbar_init(code_full + i * 8, 1); mbar_init(code_empty + i * 8, NDQ / 2); }
-        for (int i = 0; i < L::NB; ++i) { mbar_init(b_full + i * 8, 1); mbar_init(b_empty + i * 8, 2); }
-        for (int i = 0; i < 2; ++i) { mbar_init(a_full + i * 8, NDQ / 2); mbar_init(a_empty + i * 8, 2); mbar_init(done + i * 8, 2); mbar_init(acc_free + i * 8, NEPI); }
+        for (int i = 0; i < L::NB; ++i) { mbar_init(a_full + i * 8, NDQ / 2 + 1); mbar_init(b_empty + i * 8, 2); }       // the converting warps and the inputs
+        for (int i = 0; i < 2; ++i) { mbar_init(a_empty + i * 8, 2); mbar_init(done + i * 8, 2); mbar_init(acc_free + i * 8, NEPI); }
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -484,111 +505,104 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
         const uint32_t code0 = sbase + L::code + (mat * 2 + (quarter >> 1)) * 4096 + (quarter & 1) * 1024 + lane * 16;
         const uint32_t sc0 = sbase + L::code + 4 * 4096 + (mat * 2 + (quarter >> 1)) * 128 + (g * 8 + (quarter & 1) * 4) * 2;
         const uint32_t ta = tmem + TMEM_A + group * 128 + mat * 64 + ((uint32_t) (quarter * 32) << 16);      // the group's operand slot
-        uint32_t sc = 0, cph = 0, sb = 0, bph = 0, turn = 0, aph = 0;          // code ring, input ring; whose stage it is; parity of the operand slot
-        bool ok = true;
-        for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x)
+        uint32_t t0 = 0, c0 = 0;                                               // stages and code slots before this item
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x)
         {
             const ItemPos it = item_pos<DOWN>(a, item, NCT);
             if (it.n <= 0) continue;
             if (*abort_flag) break;
             const bool i8 = a.sh_i8 && it.e >= a.n_local;
-            auto code_wait = [&]() -> bool { PROBE_T0(); const bool w_ = mbar_wait(code_full + sc * 8, cph, abort_flag, a.status); if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(10); return w_; };
-            auto code_step = [&]() { if (++sc == (uint32_t) L::NCODE) { sc = 0; cph ^= 1; } };
-            auto code_release = [&]() {
+            auto code_wait = [&](uint32_t c) -> bool { PROBE_T0(); const bool w_ = pf_wait(code_full + (c % L::NCODE) * 8, (c / L::NCODE) & 1, abort_flag, a.status); if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(10); return w_; };
+            auto code_release = [&](uint32_t c) {
                 __syncwarp();
-                mbar_arrive_if(code_empty + sc * 8, lane == 0);
-                code_step();
+                mbar_arrive_if(code_empty + (c % L::NCODE) * 8, lane == 0);
             };
-            auto slot_wait = [&]() -> bool {
-                PROBE_T0(); const bool w_ = mbar_wait(a_empty + group * 8, aph ^ 1, abort_flag, a.status); if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(4);
+            auto slot_wait = [&](uint32_t t) -> bool {
+                PROBE_T0(); const bool w_ = pf_wait(a_empty + group * 8, ((t >> 1) & 1) ^ 1, abort_flag, a.status); if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(4);
                 tc_fence_after();
                 return w_;
             };
-            // both strips are stored: hand the slot to the MMA warps. One warp also makes sure that the stage's inputs are in, so that the
-            // MMA warps have one barrier to wait for.
-            auto put = [&]() -> bool {
+            // both strips are stored: hand the slot to the MMA warps
+            auto put = [&](uint32_t t) {
                 PROBE_T0();
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();
-                bool w_ = true;
-                if ((warp & 7) == 0) w_ = mbar_wait(b_full + sb * 8, bph, abort_flag, a.status);
-                __syncwarp();
-                mbar_arrive_if(a_full + group * 8, lane == 0);
+                mbar_arrive_if(a_full + (t % L::NB) * 8, lane == 0);
                 if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(9);
-                aph ^= 1;
-                return w_;
             };
-            auto run = [&](auto grouped_tag) {
+            auto run = [&](auto grouped_tag) -> bool {
                 constexpr bool GROUPED = decltype(grouped_tag)::value;
-                for (int j = 0; j < KST; ++j, turn ^= 1)
+                #pragma unroll 1
+                for (uint32_t j = (t0 ^ group) & 1; j < (uint32_t) KST; j += 2)
                 {
-                    if (turn != group) code_step();
-                    else
-                    {
-                        if (!code_wait()) { ok = false; return; }
-                        const uint32_t at = code0 + sc * L::CODE_SLOT;
-                        uint2 sp = make_uint2(0, 0);
-                        if (GROUPED) sp = lds64(sc0 + sc * L::CODE_SLOT);
-                        auto strips = [&](auto mode_tag) {
-                            constexpr Conv MODE = decltype(mode_tag)::value;
-                            uint32_t r[32], s_lo = 0, s_hi = 0;
-                            uint4 wa = lds128(at), wb = lds128(at + 2048);
-                            if (GROUPED) scale_pair(sp.x, s_lo, s_hi);
-                            convert_strip<MODE>(wa, s_lo, s_hi, r);
-                            convert_strip<MODE>(wb, s_lo, s_hi, r + 16);
-                            wa = lds128(at + 512); wb = lds128(at + 2048 + 512);
-                            if (!slot_wait()) { ok = false; return; }
-                            tmem_st_16x256(ta, r);
-                            if (GROUPED) scale_pair(sp.y, s_lo, s_hi);
-                            convert_strip<MODE>(wa, s_lo, s_hi, r);
-                            convert_strip<MODE>(wb, s_lo, s_hi, r + 16);
-                            code_release();
-                            tmem_st_16x256(ta + (16u << 16), r);
-                        };
-                        if (!GROUPED) strips(std::integral_constant<Conv, UNSCALED>());
-                        else if (__any_sync(0xffffffffu, large_scale(sp))) strips(std::integral_constant<Conv, SCALED>());
-                        else strips(std::integral_constant<Conv, FUSED>());
-                        if (!ok || !put()) { ok = false; return; }
-                    }
-                    if (++sb == (uint32_t) L::NB) { sb = 0; bph ^= 1; }
+                    const uint32_t t = t0 + j, c = c0 + j;
+                    if (!code_wait(c)) return false;
+                    const uint32_t at = code0 + (c % L::NCODE) * L::CODE_SLOT;
+                    uint2 sp = make_uint2(0, 0);
+                    if (GROUPED) sp = lds64(sc0 + (c % L::NCODE) * L::CODE_SLOT);
+                    auto strips = [&](auto mode_tag) -> bool {
+                        constexpr Conv MODE = decltype(mode_tag)::value;
+                        uint32_t r[32], s_lo = 0, s_hi = 0;
+                        uint4 wa = lds128(at), wb = lds128(at + 2048);
+                        if (GROUPED) scale_pair(sp.x, s_lo, s_hi);
+                        convert_strip<MODE>(wa, s_lo, s_hi, r);
+                        convert_strip<MODE>(wb, s_lo, s_hi, r + 16);
+                        wa = lds128(at + 512); wb = lds128(at + 2048 + 512);
+                        if (!slot_wait(t)) return false;
+                        tmem_st_16x256(ta, r);
+                        if (GROUPED) scale_pair(sp.y, s_lo, s_hi);
+                        convert_strip<MODE>(wa, s_lo, s_hi, r);
+                        convert_strip<MODE>(wb, s_lo, s_hi, r + 16);
+                        code_release(c);
+                        tmem_st_16x256(ta + (16u << 16), r);
+                        return true;
+                    };
+                    bool ok;
+                    if (!GROUPED) ok = strips(std::integral_constant<Conv, UNSCALED>());
+                    else if (__any_sync(0xffffffffu, large_scale(sp))) ok = strips(std::integral_constant<Conv, SCALED>());
+                    else ok = strips(std::integral_constant<Conv, FUSED>());
+                    if (!ok) return false;
+                    put(t);
                 }
+                return true;
             };
-            if (i8)
-            {
-                // The shared expert in the reference's int8 format (runtime/tier/tier_split.py:495-514): 2 KB units of 64 rows x 32
-                // columns, so a code slot holds 64 columns and a stage takes two. Its fp32 row scales are applied by the read-out.
-                for (int j = 0; j < KST && ok; ++j, turn ^= 1)
+            // The shared expert in the reference's int8 format (runtime/tier/tier_split.py:495-514): 2 KB units of 64 rows x 32
+            // columns, so a code slot holds 64 columns and a stage takes two. Its fp32 row scales are applied by the read-out.
+            auto run_i8 = [&]() -> bool {
+                #pragma unroll 1
+                for (uint32_t j = (t0 ^ group) & 1; j < (uint32_t) KST; j += 2)
                 {
-                    if (turn != group) { code_step(); code_step(); }
-                    else
+                    const uint32_t t = t0 + j;
+                    if (!slot_wait(t)) return false;
+                    #pragma unroll 1
+                    for (uint32_t h = 0; h < 2; ++h)
                     {
-                        if (!slot_wait()) { ok = false; break; }
-                        for (int h = 0; h < 2 && ok; ++h)
-                        {
-                            if (!code_wait()) { ok = false; break; }
-                            const uint32_t at = code0 + sc * L::CODE_SLOT;
-                            uint32_t r[16];
-                            convert_strip_i8(lds128(at), r);
-                            convert_strip_i8(lds128(at + 2048), r + 8);
-                            tmem_st_16x256_half(ta + h * 32, r);
-                            convert_strip_i8(lds128(at + 512), r);
-                            convert_strip_i8(lds128(at + 2048 + 512), r + 8);
-                            tmem_st_16x256_half(ta + h * 32 + (16u << 16), r);
-                            code_release();
-                        }
-                        if (ok && !put()) ok = false;
+                        const uint32_t c = c0 + 2 * j + h;
+                        if (!code_wait(c)) return false;
+                        const uint32_t at = code0 + (c % L::NCODE) * L::CODE_SLOT;
+                        uint32_t r[16];
+                        convert_strip_i8(lds128(at), r);
+                        convert_strip_i8(lds128(at + 2048), r + 8);
+                        tmem_st_16x256_half(ta + h * 32, r);
+                        convert_strip_i8(lds128(at + 512), r);
+                        convert_strip_i8(lds128(at + 2048 + 512), r + 8);
+                        tmem_st_16x256_half(ta + h * 32 + (16u << 16), r);
+                        code_release(c);
                     }
-                    if (++sb == (uint32_t) L::NB) { sb = 0; bph ^= 1; }
+                    put(t);
                 }
-            }
-            else if (a.grouped) run(std::true_type());
-            else run(std::false_type());
+                return true;
+            };
+            // A wait names a slot's use by its parity, so the use before must be over. The codes that were in a slot before are this group's own (the
+            // slots' number is even); an int8 stage takes two slots, but waits for its operand slot first, and int8 items come last.
+            if (!(i8 ? run_i8() : a.grouped ? run(std::true_type()) : run(std::false_type()))) break;
+            t0 += KST; c0 += i8 ? 2 * KST : KST;
         }
     }
     else if (warp == NDQ)
     {
         // ---- codes: per stage (int8: half stage) one bulk copy of 4 KB per matrix and 64-row group, lanes 0..3, and its 128 bytes of scales, lanes 4..7
-        uint32_t s = 0, ph = 0;
+        uint32_t c = 0;
         bool ok = true;
         const int blk = lane & 3, mat = blk >> 1, unit = blk & 1;
         for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x)
@@ -608,11 +622,12 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
             for (int f = 0; f < a.kfold && ok; ++f)
                 for (int j = 0; j < steps; ++j)
                 {
-                    if (!mbar_wait(code_empty + s * 8, ph ^ 1, abort_flag, a.status)) { ok = false; break; }
+                    const uint32_t s = c % L::NCODE;
+                    if (!pf_wait(code_empty + s * 8, ((c / L::NCODE) & 1) ^ 1, abort_flag, a.status)) { ok = false; break; }
                     if (lane == 0) mbar_expect_tx(code_full + s * 8, total);
                     __syncwarp();
                     if (on) bulk_g2s(dst0 + s * L::CODE_SLOT, src + (size_t) j * bytes, bytes, code_full + s * 8);
-                    if (++s == (uint32_t) L::NCODE) { s = 0; ph ^= 1; }
+                    ++c;
                 }
         }
     }
@@ -620,7 +635,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
     {
         // ---- inputs: the picks' 128 columns of a stage as two tiles of 64 columns, in boxes of 64 rows and, for the last rows, of 16, so that a
         // block with few picks brings in little more than the rows the MMAs read (n rounded up to 16)
-        uint32_t s = 0, ph = 0;
+        uint32_t t = 0;
         bool ok = true;
         for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x)
         {
@@ -631,11 +646,12 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
             const bool on = lane < 2 * nbox;
             for (int j = 0; j < KST; ++j)
             {
-                { PROBE_T0(); const bool w_ = mbar_wait(b_empty + s * 8, ph ^ 1, abort_flag, a.status); if (PROBE_ON(lane == 0)) PROBE_ADD(6); if (!w_) { ok = false; break; } }
-                if (lane == 0) mbar_expect_tx(b_full + s * 8, (uint32_t) n16 * (2 * TK * 2));
+                const uint32_t s = t % L::NB;
+                { PROBE_T0(); const bool w_ = pf_wait(b_empty + s * 8, ((t / L::NB) & 1) ^ 1, abort_flag, a.status); if (PROBE_ON(lane == 0)) PROBE_ADD(6); if (!w_) { ok = false; break; } }
+                if (lane == 0) mbar_expect_tx(a_full + s * 8, (uint32_t) n16 * (2 * TK * 2));
                 __syncwarp();
-                if (on) tma_load_2d(sbase + L::b + s * L::B_SLOT + tile * L::B_TILE + row * (TK * 2), box < nbig ? &tmap : &tmap16, j * 128 + tile * 64, it.pos0 + row, b_full + s * 8);
-                if (++s == (uint32_t) L::NB) { s = 0; ph ^= 1; }
+                if (on) tma_load_2d(sbase + L::b + s * L::B_SLOT + tile * L::B_TILE + row * (TK * 2), box < nbig ? &tmap : &tmap16, j * 128 + tile * 64, it.pos0 + row, a_full + s * 8);
+                ++t;
             }
         }
     }
@@ -647,7 +663,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
         // few picks); with two warps one's stage is under way meanwhile. All 512 columns are allocated, so the allocation starts at
         // column 0 (checked here): the addresses of the operands are plain arithmetic on loop counters.
         const uint32_t acc = warp - (NDQ + 2);
-        uint32_t sb = 0, sa = 0, aph = 0;
+        uint32_t t = 0;
         const uint64_t bdesc0 = smem_desc_sw128(sbase + L::b);
         AccSeq seq;
         bool ok = tmem == 0u;
@@ -661,17 +677,18 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
             seq.next(it.n);
             // the accumulators are free once the tiles that used their slots last have been read out
             PROBE_T0();
-            if ((seq.mask & 1) && seq.need0 && !mbar_wait(acc_free, (seq.need0 - 1) & 1, abort_flag, a.status)) ok = false;
-            if ((seq.mask & 2) && seq.need1 && !mbar_wait(acc_free + 8, (seq.need1 - 1) & 1, abort_flag, a.status)) ok = false;
+            if ((seq.mask & 1) && seq.need0 && !pf_wait(acc_free, (seq.need0 - 1) & 1, abort_flag, a.status)) ok = false;
+            if ((seq.mask & 2) && seq.need1 && !pf_wait(acc_free + 8, (seq.need1 - 1) & 1, abort_flag, a.status)) ok = false;
             if (PROBE_ON(acc == 0)) PROBE_ADD(2);
             if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
             tc_fence_after();
             const uint32_t d = seq.slot * 128 + acc * seq.up;
             const bool live = !DOWN || (int) acc < it.nmat;
-            for (int j = 0; j < KST; ++j)
+            for (int j = 0; j < KST; ++j, ++t)
             {
+                const uint32_t sb = t % L::NB, sa = t & 1;
                 bool w;
-                { PROBE_T0(); w = mbar_wait(a_full + sa * 8, aph, abort_flag, a.status); if (PROBE_ON(acc == 0)) PROBE_ADD(0); }
+                { PROBE_T0(); w = pf_wait(a_full + sb * 8, (t / L::NB) & 1, abort_flag, a.status); if (PROBE_ON(acc == 0)) PROBE_ADD(0); }
                 if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t at = TMEM_A + sa * 128 + acc * 64;
@@ -689,8 +706,6 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
                     if (j + 1 == KST) tc_commit(done + seq.slot * 8);
                 }
                 __syncwarp();
-                if (++sa == 2) { sa = 0; aph ^= 1; }
-                if (++sb == (uint32_t) L::NB) sb = 0;
             }
         }
     }
@@ -731,7 +746,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
                 float wv[2] = {0.f, 0.f};
                 #pragma unroll
                 for (int i = 0; i < 2; ++i) { const int pj = cbeg + 32 * i + lane; if (pj < n) wv[i] = __ldg(a.wt + pos0 + pj); }
-                { PROBE_T0(); const bool w_ = mbar_wait(done + seq.slot * 8, seq.done_par, abort_flag, a.status); if (PROBE_ON(threadIdx.x == (NDQ + 4) * 32)) PROBE_ADD(7); if (!w_) break; }
+                { PROBE_T0(); const bool w_ = pf_wait(done + seq.slot * 8, seq.done_par, abort_flag, a.status); if (PROBE_ON(threadIdx.x == (NDQ + 4) * 32)) PROBE_ADD(7); if (!w_) break; }
                 PROBE_T0();
                 tc_fence_after();
                 const int chp = (ch & ~63) + operand_pos(ch & 63);       // where the down GEMM expects this channel of the activations
@@ -785,33 +800,49 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
             }
             else
             {
-                { PROBE_T0(); const bool w_ = mbar_wait(done + seq.slot * 8, seq.done_par, abort_flag, a.status); if (PROBE_ON(threadIdx.x == (NDQ + 4) * 32)) PROBE_ADD(7); if (!w_) break; }
+                // lane l holds the tokens of picks l, l + 32, ... (of the last pick beyond them); fetched before the wait, and sixteen columns per
+                // step instead of eight with a load in each: 10 % of this kernel's time at 8192 rows, whose blocks of more than 64 picks keep the
+                // MMAs waiting for the read-out
+                int tok[TN / 32];
+                #pragma unroll
+                for (int i = 0; i < TN / 32; ++i) tok[i] = __ldg(a.tok + pos0 + min(32 * i + lane, n - 1));
+                { PROBE_T0(); const bool w_ = pf_wait(done + seq.slot * 8, seq.done_par, abort_flag, a.status); if (PROBE_ON(threadIdx.x == (NDQ + 4) * 32)) PROBE_ADD(7); if (!w_) break; }
                 PROBE_T0();
                 tc_fence_after();
-                // Eight columns at a time. No branch per column here either: the padding columns add 0 to the row of the block's last pick.
+                // Sixteen columns at a time; no branch per column here either: the padding columns add 0 to the row of the block's last pick.
                 const uint32_t td = tacc + half * seq.up;
                 auto read_out = [&](auto peer_tag) {
                     constexpr bool PEER = decltype(peer_tag)::value;
-                    for (int c0 = 0; c0 < n16; c0 += 8)
+                    #pragma unroll
+                    for (int i = 0; i < TN / 32; ++i)
                     {
-                        uint32_t r[8];
-                        tmem_ld8(td + c0, r);
-                        // lane j (and j + 8, ...) fetches the token of pick c0 + j while the tensor-memory load is in flight
-                        const int tj = __ldg(a.tok + pos0 + min(c0 + (lane & 7), n - 1));
-                        tmem_ld_wait();
-                        #pragma unroll
-                        for (int j = 0; j < 8; ++j)
+                        #pragma unroll 1
+                        for (int c0 = 32 * i; c0 < min(n16, 32 * i + 32); c0 += 16)
                         {
-                            const int tk = __shfl_sync(0xffffffffu, tj, j);
-                            const float v = c0 + j < n ? __uint_as_float(r[j]) * sc0 : 0.f;
-                            if (PEER)
+                            uint32_t r[16];
+                            tmem_ld16(td + c0, r);
+                            tmem_ld_wait();
+                            auto add = [&](int j, float v) {
+                                const int tk = __shfl_sync(0xffffffffu, tok[i], (c0 & 16) + j);
+                                if (PEER)
+                                {
+                                    // the row's owner may be another GPU, and up to eight GPUs add into the same addresses: the
+                                    // reduction has to be atomic at system scope (a gpu-scope one is only atomic among this GPU's threads)
+                                    const int pr = tk / a.rows_per_rank;
+                                    red_add_sys(a.out_peer[pr] + (size_t) (tk - pr * a.rows_per_rank) * a.N + ch, v);
+                                }
+                                else atomicAdd(a.out + (size_t) tk * a.N + ch, v);
+                            };
+                            if (c0 + 16 <= n)
                             {
-                                // the row's owner may be another GPU, and up to eight GPUs add into the same addresses: the
-                                // reduction has to be atomic at system scope (a gpu-scope one is only atomic among this GPU's threads)
-                                const int pr = tk / a.rows_per_rank;
-                                red_add_sys(a.out_peer[pr] + (size_t) (tk - pr * a.rows_per_rank) * a.N + ch, v);
+                                #pragma unroll
+                                for (int j = 0; j < 16; ++j) add(j, __uint_as_float(r[j]) * sc0);
                             }
-                            else atomicAdd(a.out + (size_t) tk * a.N + ch, v);
+                            else
+                            {
+                                #pragma unroll
+                                for (int j = 0; j < 16; ++j) add(j, c0 + j < n ? __uint_as_float(r[j]) * sc0 : 0.f);
+                            }
                         }
                     }
                 };
