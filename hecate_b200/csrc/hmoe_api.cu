@@ -1,6 +1,7 @@
 // The C ABI of libhecate_moe_b200.so (declared in include/hecate_moe.h) and the small stand-alone kernels: combine,
 // dequantise, status readback and the synthetic-data fill.
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include "hmoe_common.cuh"
@@ -220,17 +221,33 @@ int hmoe_short_prefill_ep(const hmoe_layer* layer, const void* x, int x_dtype, c
     return short_launch(layer, x, x_dtype, sel, rw, R, lo, n_local, act_quant, out, ws, ws_bytes, (cudaStream_t) stream, shared_row0, shared_rows);
 }
 
-// Which path serves a call of R rows: 0 decode, 1 short prefill, 2 grouped GEMMs. The short path needs the shapes whose tile
-// activations fit in registers; FORWARD_SHORT_ROWS is where the grouped GEMMs become faster
-// (measured on the benchmark layer: they cost the same from about 100 rows up because every expert's weights are converted
-// whatever its row count, the short path grows with the number of 8-pick tiles).
-static int forward_path(const hmoe_layer* L, int R, int act_quant)
+// Which path serves a call of R rows: 0 decode, 1 short prefill, 2 grouped GEMMs. The short path needs the shapes whose tile activations fit in
+// registers; it streams an expert's weights once per tile of eight picks, the grouped GEMMs once per expert (up to 128 picks), at a higher
+// price each (their conversion of the weights) and with some 40 us of permutation and gathering in front. Measured, us, short / GEMMs:
+//   6144 x 2048, 256 experts, scale groups, int4 shared: 128 rows 957 / 1300, 200 rows 1154 / 1205, 224 rows 1261 / 1241, 256 rows 1436 / 1363
+//   the same with row scales, int8 shared: 32 rows 597 / 628, 64 rows 841 / 818, 128 rows 1166 / 1037, 200 rows 1477 / 991
+//   4096 x 1024, 128 experts, row scales: 64 rows 202 / 213, 128 rows 285 / 238;  2048 x 768, 64 experts, groups: 64 rows 89 / 99, 200 rows 209 / 129
+// So the GEMMs take over once the tiles beyond the first of each expert, with the shared expert's, outweigh both: a block of the GEMMs
+// costs 1.28 (scale groups) or 1.10 (row scales) tiles, the 40 us are 11 tiles of 6144 x 2048, and the int8 shared expert adds about half a
+// tile per row to the short path. The selections are not known here: the tiles are counted for picks spread evenly over 256 router positions, the
+// most there can be, so a call whose experts get more picks than that keeps the short path for longer than it should, never the reverse. The int8
+// activation mode walks the GEMMs' weights twice and keeps the plain limit.
+static bool gemms_win(const hmoe_layer* L, int R, int n_local, bool sh8)
+{
+    if (n_local < 1) return false;                          // the GEMMs want experts
+    const double n = n_local, m = (double) R * L->topk / 256.0;
+    double p = exp(-m), cum = 0.0, extra = 0.0;             // Poisson(m) picks per expert: extra = sum over k >= 1 of P(picks > 8 k)
+    for (int c = 0; c <= 40; ++c, p *= m / c) { cum += p; if (c && c % 8 == 0) extra += 1.0 - cum; }
+    const double shared = L->sh_gate_w == nullptr ? 0.0 : sh8 ? 0.47 * R : R / 8.0;
+    const double fixed = 11.0 * (6144.0 * 2048.0) / ((double) L->H * L->I);
+    return extra * n + shared > (L->group ? 0.28 : 0.10) * n + fixed;
+}
+static int forward_path(const hmoe_layer* L, int R, int n_local, int act_quant)
 {
     const bool sh8 = L->shared_format == 1 && L->sh_gate_w != nullptr;
     if (sh8 && act_quant) return 2;           // the int8 shared expert in the int8 activation mode: only the grouped GEMMs serve it
     if (R <= MAXR) return 0;
-    // the int8 shared expert costs the short path two small launches per sixteen rows (0.43 ms at 256 rows): it hands over earlier
-    if (R <= (sh8 ? FORWARD_SHORT_ROWS_SH8 : FORWARD_SHORT_ROWS) && L->I <= 2048 && L->H <= 6144) return 1;
+    if (R <= (sh8 ? FORWARD_SHORT_ROWS_SH8 : FORWARD_SHORT_ROWS) && L->I <= 2048 && L->H <= 6144 && (act_quant || !gemms_win(L, R, n_local, sh8))) return 1;
     return 2;
 }
 int hmoe_forward_short_rows(void) { return FORWARD_SHORT_ROWS; }
@@ -249,7 +266,7 @@ int hmoe_forward(const hmoe_layer* layer, const void* x, int x_dtype, const int6
     if (!layer) return fail(HMOE_E_ARG, "hmoe_forward: null layer");
     if (R < 1) return fail(HMOE_E_ARG, "hmoe_forward: rows must be >= 1");
     if (ws_bytes < hmoe_forward_ws_bytes(R, layer->topk, n_local, layer->H, layer->I, act_quant)) return fail(HMOE_E_WS, "hmoe_forward: workspace too small");
-    switch (forward_path(layer, R, act_quant))
+    switch (forward_path(layer, R, n_local, act_quant))
     {
     case 0: return decode_launch(layer, x, x_dtype, sel, rw, R, lo, n_local, act_quant, out, ws, ws_bytes, (cudaStream_t) stream);
     case 1: return short_launch(layer, x, x_dtype, sel, rw, R, lo, n_local, act_quant, out, ws, ws_bytes, (cudaStream_t) stream);

@@ -273,9 +273,8 @@ constexpr int SHORT_MAXR = 640;               // where the grouped GEMMs catch u
 // tiles: one partial tile per local expert and for the shared expert, plus the full ones
 constexpr int SHORT_MAXT = 256 + 1 + (SHORT_MAXR * TOPK_MAX) / 8 + SHORT_MAXR / 8 + 2;
 using RouteShort = RouteT<SHORT_MAXT, unsigned short>;
-constexpr int FORWARD_SHORT_ROWS = 384;     // hmoe_forward: calls of up to this many rows take the short path (uniform routing over 256
-                                            // experts: level with the grouped GEMMs at 640 rows, 1.4 x faster at 384; skewed routing moves the crossing down)
-
-constexpr int FORWARD_SHORT_ROWS_SH8 = 256; // the same with the reference's int8 shared expert (measured: 1.69 ms against 2.2 - 2.7 ms at 256 rows, level near 384)
+// hmoe_forward: calls of more rows never take the short path, whatever its estimate says (gemms_win in hmoe_api.cu); the second limit holds for
+// layers with the reference's int8 shared expert, which costs the short path two launches per sixteen rows
+constexpr int FORWARD_SHORT_ROWS = 384, FORWARD_SHORT_ROWS_SH8 = 256;
 
 }  // namespace hmoe

@@ -137,7 +137,7 @@ def short_prefill(tables, x, sel, rw, out, ws, lo=0, n_local=None, act_quant=Fal
 
 
 def forward_short_rows():
-    """Calls of 17 .. this many rows take the short path in `forward`."""
+    """Calls of 17 .. this many rows may take the short path in `forward`; beyond, the grouped GEMMs serve them."""
     return int(lib().hmoe_forward_short_rows())
 
 
