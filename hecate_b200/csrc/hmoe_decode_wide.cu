@@ -1,0 +1,15 @@
+// The streaming kernels of layers wider than 6144 x 2048: gate_up with four chunks of 2048 columns, down with two.
+#include "hmoe_decode_stream.cuh"
+
+namespace hmoe {
+
+void launch_wide_stream(bool grouped, bool down, int grid, const void* args, cudaStream_t st, bool dependent)
+{
+    const DecodeArgs& a = *(const DecodeArgs*) args;
+    if (grouped && down) launch_stream<true, false, true, 2>(grid, a, st, dependent);
+    else if (grouped) launch_stream<true, false, false, 4>(grid, a, st, dependent);
+    else if (down) launch_stream<false, false, true, 2>(grid, a, st, dependent);
+    else launch_stream<false, false, false, 4>(grid, a, st, dependent);
+}
+
+}  // namespace hmoe

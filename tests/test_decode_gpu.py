@@ -135,6 +135,14 @@ def test_single_token_full_width(oracle, dev, aq):
     assert (e[0] < MAX_REL and e[1] < MEAN_ABS) if aq else e[2] < NORM_REL_EXACT, e
 
 
+@pytest.mark.parametrize("group,R", [(0, 1), (128, 11), (0, 16)])
+@pytest.mark.parametrize("H,I", [(6272, 256), (8192, 384), (512, 2176), (384, 4096), (8320, 256), (256, 4224)])
+def test_wide_shapes(oracle, dev, H, I, group, R):
+    """The widest chunk counts of the streaming kernels (partly filled and full), and the first widths beyond them."""
+    (got,), ref = run_case(oracle, dev, H, I, 8, R, group, True, False, seed=9)
+    assert errors(got, ref)[2] < NORM_REL_EXACT, errors(got, ref)
+
+
 @pytest.mark.parametrize("H,I", [(6272, 256), (512, 2176)])
 def test_shapes_beyond_the_register_resident_path(oracle, dev, H, I):
     """H > 6144 or I > 2048: a tile's activation fragments no longer fit in registers and the call takes the kernels that
