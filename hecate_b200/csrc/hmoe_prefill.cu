@@ -447,8 +447,8 @@ __device__ __forceinline__ ItemPos item_pos(const GemmArgs& a, int item, int nct
     const int rs = item / nct;
     it.ct = item - rs * nct;
     const int rb = a.nsub == 1 ? rs : rs / a.nsub, sub = a.nsub == 1 ? 0 : rs - rb * a.nsub;
-    const int4 r = __ldg((const int4*) a.rbt + rb);
-    it.e = r.x; it.pos0 = r.y + sub * TN; it.n = min(r.z - sub * TN, TN);
+    const int* r = a.rbt + 4 * (size_t) rb;                 // word by word: a caller's table (hmoe_prefill_sorted) need not start on 16 bytes
+    it.e = __ldg(r); it.pos0 = __ldg(r + 1) + sub * TN; it.n = min(__ldg(r + 2) - sub * TN, TN);
     it.nmat = DOWN ? (2 * it.ct + 1 < a.N / TM ? 2 : 1) : 2;
     return it;
 }

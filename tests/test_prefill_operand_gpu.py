@@ -50,8 +50,10 @@ def test_scales_beyond_the_fused_conversion(oracle):
     assert np.isfinite(e[2]) and e[2] < NORM_REL, e
 
 
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
 @pytest.mark.parametrize("picks", [128, 129, 200, 256])
-def test_row_blocks_of_a_caller_up_to_256_picks(oracle, picks):
+def test_row_blocks_of_a_caller_up_to_256_picks(oracle, picks, offset):
+    """The table may start on any 4-byte boundary (a part of a larger int32 buffer)."""
     import torch
     from hecate_b200 import moe
     dev = torch.device("cuda:0")
@@ -69,7 +71,10 @@ def test_row_blocks_of_a_caller_up_to_256_picks(oracle, picks):
     tok = torch.cat([torch.arange(picks), torch.arange(5)]).to(torch.int32).to(dev)
     eid = torch.cat([torch.zeros(picks), torch.ones(5)]).to(torch.int32).to(dev)
     wt = torch.full((picks + 5,), 0.125, dtype=torch.float32, device=dev)
-    rbt = torch.tensor([[0, 0, picks, 0], [1, picks, 5, 0]], dtype=torch.int32, device=dev)
+    buf = torch.zeros(8 + offset, dtype=torch.int32, device=dev)
+    rbt = buf[offset:].view(2, 4)
+    rbt.copy_(torch.tensor([[0, 0, picks, 0], [1, picks, 5, 0]]))
+    assert rbt.data_ptr() % 16 == 4 * offset
     out = torch.zeros(picks, H, device=dev)
     t = tabs.tabs
     moe.moe4t_forward(torch.from_numpy(x).to(dev), tok, eid, wt, rbt, t["gate_w"], t["up_w"], t["down_w"], t["gate_s"], t["up_s"], t["down_s"],
