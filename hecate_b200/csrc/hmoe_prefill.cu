@@ -38,6 +38,7 @@
 #include <type_traits>
 #include "hmoe_common.cuh"
 #include "hmoe_internal.h"
+#include "hmoe_prefill_order.h"
 
 namespace hmoe {
 namespace {
@@ -407,13 +408,13 @@ __device__ __forceinline__ void scale_pair(uint32_t bf2, uint32_t& s_lo, uint32_
 // memory's full rate; five or seven slots measured no faster), inputs NB stages ahead; the converted weights never come here.
 struct PfSmem
 {
-    static constexpr int NCODE = 4, NB = 4;                  // powers of two: a running stage number gives slot and parity
+    static constexpr int NCODE = PF_NCODE, NB = 4;           // powers of two: a running stage number gives slot and parity
     static constexpr int CODE_SLOT = 4 * 4096 + 4 * 128;
     static constexpr int B_TILE = TN * TK * 2, B_SLOT = 2 * B_TILE;
     static constexpr int b = 0;
     static constexpr int code = NB * B_SLOT;
-    static constexpr int bars = code + NCODE * CODE_SLOT;   // code_full, code_empty [NCODE], b_empty, a_full [NB], a_empty, done, acc_free [2]
-    static constexpr int misc = bars + (2 * NCODE + 2 * NB + 6) * 8;
+    static constexpr int bars = code + NCODE * CODE_SLOT;   // code_full, code_empty [NCODE], b_empty, a_full [NB], a_empty, done, acc_free [2], i8_done
+    static constexpr int misc = bars + (2 * NCODE + 2 * NB + 7) * 8 + 8;
     static constexpr int total = misc + 32 + 1024;          // + slack to align the base to 1024
 };
 // tensor memory: columns 0..255 accumulators (two slots of 128: a block of up to 64 picks takes one slot for its two accumulators, a larger
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
     const uint32_t sbase = (raw + 1023u) & ~1023u;
     unsigned char* smem = smem_raw + (sbase - raw);
     const uint32_t code_full = sbase + L::bars, code_empty = code_full + L::NCODE * 8, b_empty = code_empty + L::NCODE * 8, a_full = b_empty + L::NB * 8,
-                   a_empty = a_full + L::NB * 8, done = a_empty + 16, acc_free = done + 16;
+                   a_empty = a_full + L::NB * 8, done = a_empty + 16, acc_free = done + 16, i8_done = acc_free + 16;
     uint32_t* tmem_slot = (uint32_t*) (smem + L::misc);
     volatile int* abort_flag = (volatile int*) (smem + L::misc + 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -473,6 +474,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
         for (int i = 0; i < L::NCODE; ++i) { mbar_init(code_full + i * 8, 1); mbar_init(code_empty + i * 8, NDQ / 2); }
         for (int i = 0; i < L::NB; ++i) { mbar_init(a_full + i * 8, NDQ / 2 + 1); mbar_init(b_empty + i * 8, 2); }       // the converting warps and the inputs
         for (int i = 0; i < 2; ++i) { mbar_init(a_empty + i * 8, 2); mbar_init(done + i * 8, 2); mbar_init(acc_free + i * 8, NEPI); }
+        mbar_init(i8_done, NDQ);
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -506,6 +508,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
         const uint32_t sc0 = sbase + L::code + 4 * 4096 + (mat * 2 + (quarter >> 1)) * 128 + (g * 8 + (quarter & 1) * 4) * 2;
         const uint32_t ta = tmem + TMEM_A + group * 128 + mat * 64 + ((uint32_t) (quarter * 32) << 16);      // the group's operand slot
         uint32_t t0 = 0, c0 = 0;                                               // stages and code slots before this item
+        CodeOrder order;
         for (int item = blockIdx.x; item < nitems; item += gridDim.x)
         {
             const ItemPos it = item_pos<DOWN>(a, item, NCT);
@@ -593,8 +596,12 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
                 }
                 return true;
             };
-            // A wait names a slot's use by its parity, so the use before must be over. The codes that were in a slot before are this group's own (the
-            // slots' number is even); an int8 stage takes two slots, but waits for its operand slot first, and int8 items come last.
+            if (order.wait_first(i8))
+            {
+                __syncwarp();
+                mbar_arrive_if(i8_done, lane == 0);
+                if (!pf_wait(i8_done, (order.crossings - 1) & 1, abort_flag, a.status)) break;
+            }
             if (!(i8 ? run_i8() : a.grouped ? run(std::true_type()) : run(std::false_type()))) break;
             t0 += KST; c0 += i8 ? 2 * KST : KST;
         }

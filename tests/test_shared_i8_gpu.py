@@ -94,3 +94,48 @@ def test_int8_shared_expert_in_prefill(oracle, H, I, R, group):
     moe.forward(tabs, up(x[:ns]), up(sel[:ns]), up(rw[:ns]), yq, wsf, act_quant=True)
     moe.prefill(tabs, up(x[:ns]), up(sel[:ns]), up(rw[:ns]), yp, moe.prefill_workspace(ns, 8, E, H, I, dev, act_quant=True), act_quant=True)
     assert moe.ws_status(wsf) == 0 and errors(yq.cpu().numpy(), yp.cpu().numpy())[2] < 1e-5       # the same kernels; the sums' order differs
+
+
+@pytest.mark.parametrize("group", [0, 128])
+@pytest.mark.parametrize("H,I", [(384, 256), (256, 384), (512, 640)])
+@pytest.mark.parametrize("every", [1, 4])
+def test_int8_shared_expert_anywhere_in_a_caller_table(oracle, H, I, group, every):
+    """hmoe_prefill_sorted with the int8 shared expert's blocks first and among the routed ones (which the library's own permutation puts in
+    front): an int8 stage takes two code slots, so what follows it finds the slots in another turn. Odd and even numbers of stages per item."""
+    import ctypes as C
+    import torch
+    from hecate_b200 import _lib, moe
+    dev = torch.device("cuda:0")
+    E, R = 8, 60
+    hl = HostLayer(9, 0, H, I, range(E), group, False)
+    base = hl.upload(dev)
+    ex8 = _int8_expert(13, H, I)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+    shared = tuple(up(layout.pack_i8(c)) for c, _ in ex8) + tuple(up(s) for _, s in ex8)
+    tabs = moe.ExpertTables(H, I, 8, *[base.keep[i] for i in range(6)], group=group, shared=shared, device=dev, shared_i8=True)
+    x = synth.activations(3, 0, R, H).astype(np.float16); sel, rw = random_routing(4, R, E)
+    ex, _ = hl.oracle_experts(oracle)
+    ref = oracle.moe_forward(H, I, group, x, sel, rw, 0, ex, None, mode=1).astype(np.float64) + _shared_exact(x, ex8)
+    # blocks of up to three picks; behind every `every` routed blocks, and in front of all, one of the shared expert
+    routed = [(e, [(int(r), float(rw[r, k])) for r in range(R) for k in range(8) if sel[r, k] == e]) for e in range(E)]
+    routed = [(e, p[i:i + 3]) for e, p in routed for i in range(0, len(p), 3)]
+    extra = [(E, [(r, 1.0) for r in range(i, min(i + every, R))]) for i in range(0, R, every)]
+    blocks = [extra.pop(0)]
+    for i, b in enumerate(routed):
+        blocks.append(b)
+        if i % every == every - 1 and extra:
+            blocks.append(extra.pop(0))
+    blocks += extra
+    tok, wt, rbt = [], [], []
+    for e, picks in blocks:
+        rbt.append((e, len(tok), len(picks), 0))
+        tok += [r for r, _ in picks]; wt += [w for _, w in picks]
+    tok, wt, rbt = np.array(tok, dtype=np.int32), np.array(wt, dtype=np.float32), np.array(rbt, dtype=np.int32)
+    lib, st, out = moe.lib(), tabs.struct(), torch.zeros(R, H, device=dev)
+    n = lib.hmoe_prefill_sorted_ws_bytes(C.c_int(len(tok)), C.c_int(H), C.c_int(I), C.c_int(0))
+    ws = torch.zeros(n, dtype=torch.uint8, device=dev)
+    xs, ts, wts, rs = up(x), up(tok), up(wt), up(rbt)
+    _lib.check(lib.hmoe_prefill_sorted(C.byref(st), _lib.vp(xs), C.c_int(_lib.F16), _lib.vp(ts), _lib.vp(wts), _lib.vp(rs), C.c_int(len(rbt)),
+                                       C.c_int(len(tok)), C.c_int(E), C.c_int(0), _lib.vp(out), _lib.vp(ws), C.c_size_t(n), moe._stream(dev)))
+    assert moe.ws_status(ws) == 0
+    assert errors(out.cpu().numpy(), ref)[2] < NORM_REL_EXACT, errors(out.cpu().numpy(), ref)
