@@ -256,8 +256,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_gate_up_kernel(const Decod
     const int P = rt->ntiles * NG;
     const int p0 = (int) ((long long) P * blockIdx.x / gridDim.x), p1 = (int) ((long long) P * (blockIdx.x + 1) / gridDim.x);
     const int mat = warp >> 3, kw = warp & 7, g = lane >> 2, q = lane & 3;
-    // fill cursor of this warp: the next stage to request is stage f_s of item (f_tile, f_gr); f_src = its matrix's packed codes
-    int f_tile = p0 / NG, f_gr = p0 % NG, f_s = 0, f_left = p1 - p0;
+    // fill cursor of this warp: the next stage to request is stage f_s of item (f_tile, f_gr); f_src = its matrix's packed codes. A slot is one of the
+    // stages in which the warp has columns (the last one of an item, when it is not full, has none for some warps): a slot that were passed over
+    // unfilled would not turn its barrier's phase.
+    int f_tile = p0 / NG, f_gr = p0 % NG, f_s = 0, f_left = 2 * kw < KB ? p1 - p0 : 0;
     auto item_src = [&](int tile, int gr) {
         const int e = rt->expert[tile];
         return (const char*) (e >= 0 ? (const void*) (mat ? a.up_w[e] : a.gate_w[e]) : (mat ? a.sh_uw : a.sh_gw)) + (size_t) gr * KB * 2048;
@@ -265,14 +267,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_gate_up_kernel(const Decod
     const char* f_src = p0 < p1 ? item_src(f_tile, f_gr) : nullptr;      // looked up when the cursor enters an item, used a stage later
     auto fill_next = [&](uint32_t slot) {
         if (f_left <= 0) return;
-        const int kb = 16 * f_s + 2 * kw;
-        if (kb < KB)
-        {
-            const uint32_t bar = full0 + (slot * CW + warp) * 8;
-            mbar_expect_tx(bar, 4096);
-            bulk_g2s(ring + slot * STAGE_BYTES + warp * 4096, f_src + (size_t) kb * 2048, 4096, bar);
-        }
-        if (++f_s == S)
+        const uint32_t bar = full0 + (slot * CW + warp) * 8;
+        mbar_expect_tx(bar, 4096);
+        bulk_g2s(ring + slot * STAGE_BYTES + warp * 4096, f_src + (size_t) (16 * f_s + 2 * kw) * 2048, 4096, bar);
+        if (16 * ++f_s + 2 * kw >= KB)
         {
             f_s = 0; --f_left;
             if (++f_gr == NG) { f_gr = 0; ++f_tile; }
@@ -371,11 +369,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_gate_up_kernel(const Decod
                 {
                     if (!mbar_wait(full0 + (st * CW + warp) * 8, par, abort_flag, a.status)) { alive = false; break; }
                     consume_group<GROUPED, Q8>(ring + st * STAGE_BYTES + warp * 4096, pc.bx, pc.sc, pc.sx[0], pc.sx[1], acc, lane);
+                    __syncwarp();
+                    if (lane == 0) fill_next(st);
+                    if (++st == NSTAGE) { st = 0; par ^= 1; }
                 }
-                __syncwarp();
-                if (lane == 0) fill_next(st);
                 if (s == 0 && have_prev) { finish_item(prev, prev_idx); have_prev = false; }
-                if (++st == NSTAGE) { st = 0; par ^= 1; }
                 pc = pn;
             }
             if (!alive) break;

@@ -151,6 +151,17 @@ def test_shapes_beyond_the_register_resident_path(oracle, dev, H, I):
     assert int8_close(errors(got, ref)), errors(got, ref)
 
 
+@pytest.mark.parametrize("H,I,aq", [(6400, 1024, True), (6272, 1152, True), (4352, 2176, True), (8448, 1024, False), (1152, 4224, False), (1152, 4224, True)])
+def test_wide_shapes_with_several_items_per_block(oracle, dev, H, I, aq):
+    """H is no multiple of 1024, so the last stage of an item leaves some warps without columns, and a block goes through several items: the warps' rings
+    must not count the stages they have no part in. (These layers take the kernels that fetch activations stage by stage.)"""
+    for group in (0, 128):
+        outs, ref = run_case(oracle, dev, H, I, 24, 16, group, True, aq, seed=11, calls=2)
+        for got in outs:
+            e = errors(got, ref)
+            assert int8_close(e) if aq else e[2] < NORM_REL_EXACT, (group, e)
+
+
 @pytest.mark.parametrize("R,H,I,E,aq", [(16, 6144, 2048, 32, False), (5, 6144, 2048, 32, True), (1, 512, 256, 32, True), (13, 1024, 256, 64, False)])
 def test_router_decode_in_one_call_equals_the_two_calls(oracle, dev, R, H, I, E, aq):
     """hmoe_router_decode (the router's launch also does the decode call's set-up step) against hmoe_router followed by
