@@ -301,18 +301,21 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr)
     return v;
 }
 
-// Bounded wait like mbar_wait in fewer instructions (these kernels' converting warps leave few issue slots to spare). The first try is a short
-// one: parked for long from the first try on, the thread wakes up later (measured: 64 to 2048 rows 3 to 7 % slower).
+// Bounded wait of a whole warp, like mbar_wait in fewer instructions (these kernels' converting warps leave few issue slots to spare). Every lane leaves it
+// with the same answer: what follows are instructions of the whole warp (tensor-memory loads and stores, votes, shuffles), which lanes that gave up
+// must not miss. The first try is a short one: parked for long from the first try on, the thread wakes up later (measured: 64 to 2048 rows 3 to 7 %
+// slower).
 __device__ __forceinline__ bool pf_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned* status)
 {
-    if (mbar_try(bar, parity)) return true;
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
     unsigned long long t0 = 0;
-    while (!mbar_try_hint(bar, parity, 20000u))
+    while (!__all_sync(0xffffffffu, mbar_try_hint(bar, parity, 20000u)))
     {
-        if (*abort_flag) return false;
         const unsigned long long now = globaltimer_ns();
+        const bool late = t0 != 0 && now - t0 > 1000000000ull;
         if (t0 == 0) t0 = now;
-        else if (now - t0 > 1000000000ull) { *abort_flag = 1; if (status) atomicOr(status, ST_WAIT_TIMEOUT); return false; }
+        if (late) { *abort_flag = 1; if (status) atomicOr(status, ST_WAIT_TIMEOUT); }
+        if (__any_sync(0xffffffffu, late || *abort_flag)) return false;
     }
     return true;
 }
@@ -513,7 +516,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
         {
             const ItemPos it = item_pos<DOWN>(a, item, NCT);
             if (it.n <= 0) continue;
-            if (*abort_flag) break;
+            if (__any_sync(0xffffffffu, *abort_flag)) break;
             const bool i8 = a.sh_i8 && it.e >= a.n_local;
             auto code_wait = [&](uint32_t c) -> bool { PROBE_T0(); const bool w_ = pf_wait(code_full + (c % L::NCODE) * 8, (c / L::NCODE) & 1, abort_flag, a.status); if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(10); return w_; };
             auto code_release = [&](uint32_t c) {
@@ -530,6 +533,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
                 PROBE_T0();
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();
+                __syncwarp();
                 mbar_arrive_if(a_full + (t % L::NB) * 8, lane == 0);
                 if (PROBE_ON(threadIdx.x == 0)) PROBE_ADD(9);
             };
@@ -687,7 +691,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
             if ((seq.mask & 1) && seq.need0 && !pf_wait(acc_free, (seq.need0 - 1) & 1, abort_flag, a.status)) ok = false;
             if ((seq.mask & 2) && seq.need1 && !pf_wait(acc_free + 8, (seq.need1 - 1) & 1, abort_flag, a.status)) ok = false;
             if (PROBE_ON(acc == 0)) PROBE_ADD(2);
-            if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+            if (!ok) break;
             tc_fence_after();
             const uint32_t d = seq.slot * 128 + acc * seq.up;
             const bool live = !DOWN || (int) acc < it.nmat;
@@ -696,7 +700,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
                 const uint32_t sb = t % L::NB, sa = t & 1;
                 bool w;
                 { PROBE_T0(); w = pf_wait(a_full + sb * 8, (t / L::NB) & 1, abort_flag, a.status); if (PROBE_ON(acc == 0)) PROBE_ADD(0); }
-                if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
+                if (!w) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t at = TMEM_A + sa * 128 + acc * 64;
                 const uint64_t bd = bdesc0 + sb * (L::B_SLOT >> 4);
@@ -730,7 +734,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
         {
             const ItemPos it = item_pos<DOWN>(a, item, NCT);
             if (it.n <= 0) continue;
-            if (*abort_flag) break;
+            if (__any_sync(0xffffffffu, *abort_flag)) break;
             const int e = it.e, pos0 = it.pos0, n = it.n, n16 = (n + 15) & ~15;
             seq.next(n);
             const bool live = !DOWN || half < it.nmat;
