@@ -80,6 +80,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (status) atomicOr(status, ST_WAIT_TIMEOUT);
     return false;
 }
+// A block in which a wait gave up may have copies in flight into its shared memory: it leaves them time to land (2 ms) before it returns. Called by the
+// whole block behind a barrier.
+__device__ __forceinline__ void abort_drain(volatile int* abort_flag)
+{
+    if (*abort_flag == 0) return;
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) ;
+}
 // Diagnostic build (-DHMOE_PROBE_TIMELINE): kernels of the decode chain stamp the global timer at a few points (earliest and latest
 // over the blocks); every source file has its own table and reader. Not part of the normal build.
 #ifdef HMOE_PROBE_TIMELINE

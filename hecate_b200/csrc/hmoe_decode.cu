@@ -407,6 +407,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_gate_up_kernel(const Decod
         if (alive && have_prev) finish_item(prev, prev_idx);
     }
     __syncthreads();
+    abort_drain(abort_flag);
 }
 
 // down's ring is shared by the block and refilled by whichever warp frees a stage last: after its last read of stage number `it` a warp bumps the
@@ -553,6 +554,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_down_kernel(const DecodeAr
         }
     }
     __syncthreads();
+    abort_drain(abort_flag);
 }
 
 }  // namespace

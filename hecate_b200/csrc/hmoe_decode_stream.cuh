@@ -443,6 +443,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_stream_kernel(const Decode
     }
     else if (DOWN) { pdl_wait(); pdl_launch_dependents(); }
     __syncthreads();
+    abort_drain(abort_flag);
     TL_MAX(DOWN ? 9 : 1);
     if (DOWN && a.ep.world > 0) ep_tail_combine(a.ep, *a.gen_ptr, a.slot_stride, a.H);
 }

@@ -873,12 +873,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_gemm_kernel(const __gri
 #endif
     tc_fence_before();
     __syncthreads();
-    if (*abort_flag && threadIdx.x == 0)
-    {
-        // a wait gave up: copies may still be in flight into this block's shared memory; leave them time to land
-        const unsigned long long t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 2000000ull) ;
-    }
+    abort_drain(abort_flag);
     __syncthreads();
     if (warp == NDQ + 2)
     {
