@@ -223,24 +223,24 @@ int hmoe_short_prefill_ep(const hmoe_layer* layer, const void* x, int x_dtype, c
 
 // Which path serves a call of R rows: 0 decode, 1 short prefill, 2 grouped GEMMs. The short path needs the shapes whose tile activations fit in
 // registers; it streams an expert's weights once per tile of eight picks, the grouped GEMMs once per expert (up to 128 picks), at a higher
-// price each (their conversion of the weights) and with some 40 us of permutation and gathering in front. Measured, us, short / GEMMs:
-//   6144 x 2048, 256 experts, scale groups, int4 shared: 128 rows 957 / 1300, 200 rows 1154 / 1205, 224 rows 1261 / 1241, 256 rows 1436 / 1363
-//   the same with row scales, int8 shared: 32 rows 597 / 628, 64 rows 841 / 818, 128 rows 1166 / 1037, 200 rows 1477 / 991
-//   4096 x 1024, 128 experts, row scales: 64 rows 202 / 213, 128 rows 285 / 238;  2048 x 768, 64 experts, groups: 64 rows 89 / 99, 200 rows 209 / 129
+// price each (their conversion of the weights) and with some 40 us of permutation and gathering in front. Measured, us, short / GEMMs, row scales:
+//   6144 x 2048, 256 experts, int8 shared: 32 rows 597 / 628, 64 rows 841 / 818, 128 rows 1166 / 1037, 200 rows 1477 / 991
+//   4096 x 1024, 128 experts: 64 rows 202 / 213, 128 rows 285 / 238;  int4 shared, 6144 x 2048, 256 experts: 160 rows 1023 / 954, 256 rows 1478 / 992
 // So the GEMMs take over once the tiles beyond the first of each expert, with the shared expert's, outweigh both: a block of the GEMMs
-// costs 1.28 (scale groups) or 1.10 (row scales) tiles, the 40 us are 11 tiles of 6144 x 2048, and the int8 shared expert adds about half a
+// costs 1.10 tiles, the 40 us are 11 tiles of 6144 x 2048, and the int8 shared expert adds about half a
 // tile per row to the short path. The selections are not known here: the tiles are counted for picks spread evenly over 256 router positions, the
 // most there can be, so a call whose experts get more picks than that keeps the short path for longer than it should, never the reverse. The int8
-// activation mode walks the GEMMs' weights twice and keeps the plain limit.
+// activation mode walks the GEMMs' weights twice and keeps the plain limit. So do layers with scale groups: the short path applies the scales to fp32 sums, the
+// GEMMs to the fp16 weights, which is exact only from 2^-17 to below 8192.
 static bool gemms_win(const hmoe_layer* L, int R, int n_local, bool sh8)
 {
-    if (n_local < 1) return false;                          // the GEMMs want experts
+    if (n_local < 1 || L->group) return false;              // the GEMMs want experts
     const double n = n_local, m = (double) R * L->topk / 256.0;
     double p = exp(-m), cum = 0.0, extra = 0.0;             // Poisson(m) picks per expert: extra = sum over k >= 1 of P(picks > 8 k)
     for (int c = 0; c <= 40; ++c, p *= m / c) { cum += p; if (c && c % 8 == 0) extra += 1.0 - cum; }
     const double shared = L->sh_gate_w == nullptr ? 0.0 : sh8 ? 0.47 * R : R / 8.0;
     const double fixed = 11.0 * (6144.0 * 2048.0) / ((double) L->H * L->I);
-    return extra * n + shared > (L->group ? 0.28 : 0.10) * n + fixed;
+    return extra * n + shared > 0.10 * n + fixed;
 }
 static int forward_path(const hmoe_layer* L, int R, int n_local, int act_quant)
 {

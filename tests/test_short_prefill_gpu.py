@@ -218,17 +218,14 @@ def test_forward_reuses_one_workspace_across_paths(oracle, dev):
             assert (e[0] < MAX_REL and e[1] < MEAN_ABS) if aq else e[2] < NORM_REL_EXACT, (aq, R, e)
 
 
-@pytest.mark.parametrize("R,group,shared,lo,n,act", [(384, 128, "int4", 0, 64, "bf16"), (300, 128, "none", 0, 64, "fp16"), (260, 0, "none", 32, 48, "bf16"),
-                                                     (60, 0, "int8", 0, 64, "fp16"), (384, 0, "int4", 60, 9, "bf16")])
-def test_forward_hands_over_to_the_grouped_gemms(dev, R, group, shared, lo, n, act):
-    """Rows at which forward leaves the short path before its row limit (counted by the launches): the same result as the short path. Both
-    round the SiLU product to fp16 once (2.8e-4 from the layer in 64 bits), so they differ by at most twice that."""
+def _random_layer(dev, seed, n, group, shared):
+    """6144 x 2048 with n random experts on the device: their tables and the generator."""
     import torch
     from hecate_b200 import moe
-    H, I, E = 6144, 2048, 64
-    g = torch.Generator(device=dev); g.manual_seed(R)
+    H, I = 6144, 2048
+    g = torch.Generator(device=dev); g.manual_seed(seed)
     w = torch.empty(n + 1, 3, I * H // 2, dtype=torch.uint8, device=dev)
-    moe.fill_bytes(w, 5, R)
+    moe.fill_bytes(w, 5, seed)
     logn = lambda *s: (torch.randn(*s, device=dev, generator=g) * 0.5 - 4.0).exp()
     if group:
         sc = [logn(n + 1, N // 64, K // 128, 64).to(torch.bfloat16) for N, K in ((I, H), (I, H), (H, I))]
@@ -239,18 +236,55 @@ def test_forward_hands_over_to_the_grouped_gemms(dev, R, group, shared, lo, n, a
         sh = (w[n, 0], w[n, 1], w[n, 2], sc[0][n], sc[1][n], sc[2][n])
     elif shared == "int8":
         q = torch.empty(3, H * I, dtype=torch.uint8, device=dev)
-        moe.fill_bytes(q, 6, R)
+        moe.fill_bytes(q, 6, seed)
         sh = (q[0], q[1], q[2], *(logn(N) / 16 for N in (I, I, H)))
     tabs = moe.ExpertTables(H, I, 8, *[list(w[:n, k]) for k in range(3)], *[list(sc[k][:n]) for k in range(3)], group=group, shared=sh, device=dev,
                             shared_i8=shared == "int8")
+    return tabs, sc, g
+
+
+def _forward_and_short(dev, tabs, g, R, E, lo, act):
+    """Both calls on the same random inputs, and the launches of the first."""
+    import torch
+    from hecate_b200 import moe
+    H, I, n = tabs.H, tabs.I, tabs.n
     x = torch.randn(R, H, device=dev, generator=g).to(torch.bfloat16 if act == "bf16" else torch.float16)
-    sel = torch.rand(R, max(E, lo + n), device=dev, generator=g).topk(8, dim=1).indices
+    sel = torch.rand(R, E, device=dev, generator=g).topk(8, dim=1).indices
     rw = torch.rand(R, 8, device=dev, generator=g).half()
     got, want = torch.zeros(R, H, device=dev), torch.zeros(R, H, device=dev)
     ws, ws2 = moe.forward_workspace(R, 8, n, H, I, dev), moe.short_prefill_workspace(R, H, I, 8, dev)
     before = moe.launch_count()
     moe.forward(tabs, x, sel, rw, got, ws, lo=lo)
-    assert moe.launch_count() - before == 6                 # permutation (3), gather, two GEMMs
+    launches = moe.launch_count() - before
     moe.short_prefill(tabs, x, sel, rw, want, ws2, lo=lo)
     assert moe.ws_status(ws) == 0 and moe.ws_status(ws2) == 0
+    return got, want, launches
+
+
+@pytest.mark.parametrize("R,shared,lo,n,act", [(384, "int4", 0, 64, "bf16"), (300, "none", 0, 64, "fp16"), (260, "none", 32, 48, "bf16"),
+                                               (60, "int8", 0, 64, "fp16"), (384, "int4", 60, 9, "bf16")])
+def test_forward_hands_over_to_the_grouped_gemms(dev, R, shared, lo, n, act):
+    """Rows at which forward leaves the short path before its row limit (counted by the launches): the same result as the short path. Both
+    round the SiLU product to fp16 once (2.8e-4 from the layer in 64 bits), so they differ by at most twice that."""
+    tabs, _, g = _random_layer(dev, R, n, 0, shared)
+    got, want, launches = _forward_and_short(dev, tabs, g, R, max(64, lo + n), lo, act)
+    assert launches == 6                                    # permutation (3), gather, two GEMMs
     assert float((got - want).double().norm() / want.double().norm()) < 5.6e-4
+
+
+@pytest.mark.parametrize("scales", ["large", "small"])
+@pytest.mark.parametrize("R,shared", [(384, "int4"), (300, "none"), (256, "none")])
+def test_forward_keeps_scale_groups_in_32_bits(dev, R, shared, scales):
+    """Scales that the GEMMs' fp16 weights cannot hold (7 x 12288 is beyond fp16; 4e-7 keeps three bits there): up to its row limit forward gives what the
+    short path gives, which applies them to fp32 sums. The two calls add the gate and up sums in different orders, so a SiLU product may round
+    to the neighbouring fp16 value: 2^-10 of it at most, and so of a row."""
+    import torch
+    tabs, sc, g = _random_layer(dev, R, 64, 128, shared)
+    if scales == "large":
+        sc[2][1:64:3, :, 5] = 12288.0
+    else:
+        sc[2].fill_(1.3671875 * 2.0 ** -22)
+    got, want, _ = _forward_and_short(dev, tabs, g, R, 64, 0, "bf16")
+    assert bool(torch.isfinite(got).all())
+    err = (got - want).double().norm(dim=1) / want.double().norm(dim=1)
+    assert float(err.max()) < 2.0 ** -10, float(err.max())
