@@ -616,7 +616,8 @@ int decode_phase_times(float* ms3)
 
 // Shapes of the streaming kernels: a tile's activation fragments (16 registers per 2048 columns) have to fit into registers, in the int8 mode with
 // their scales beside them. (Measured against the kernels that fetch them stage by stage, us per decode step: 7168 x 2560, 64 experts, 6 rows
-// 286 -> 233; 8192 x 1536, 16 rows 344 -> 261; 4096 x 3072, 8 rows 245 -> 182.)
+// 286 -> 233; 8192 x 1536, 16 rows 344 -> 261; 4096 x 3072, 8 rows 245 -> 182. Sixteen partial sums per result here, eight there: the same distance
+// from the layer in 64 bits, 1.64e-4 to 2.01e-4 over seven wide shapes and formats at 1, 6 and 16 rows, differing in the fourth digit either way.)
 static bool stream_shape(int H, int I, int act_quant) { return act_quant ? H <= 6144 && I <= 2048 : H <= 8192 && I <= 4096; }
 
 template <bool G, bool Q>
@@ -638,7 +639,7 @@ static void launch_pair(int grid, const DecodeArgs& a, int R, cudaStream_t st)
     else launch_wide_stream(G, false, grid, &a, st, !g_prof);
     if (g_prof) cudaEventRecord(ev[2], st);
     if (!resident) decode_down_kernel<G, Q><<<grid, NTHREADS, SmemLayout::total, st>>>(a, R);
-    else if (a.I <= 2048) launch_stream<G, Q, true, 1>(grid, a, st, !g_prof);
+    else if (a.I <= 2048 && a.H <= 6144) launch_stream<G, Q, true, 1>(grid, a, st, !g_prof);
     else launch_wide_stream(G, true, grid, &a, st, !g_prof);
     if (g_prof) { cudaEventRecord(ev[3], st); ++g_prof_calls; }
 }

@@ -203,7 +203,8 @@ struct StreamSmem
     static constexpr int total = flags + 16;
 };
 
-template <bool GROUPED, bool Q8, bool DOWN, int KC, typename RT = Route>
+// WIDE: layers wider than 6144 x 2048, whose SiLU has always been computed with expf, as in the int8 mode.
+template <bool GROUPED, bool Q8, bool DOWN, int KC, typename RT = Route, bool WIDE = false>
 __global__ void __launch_bounds__(NTHREADS, 1) decode_stream_kernel(const DecodeArgs a)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -328,11 +329,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_stream_kernel(const Decode
                         const float2 u0 = __ldcg((const float2*) (gp + a.I)), u1 = __ldcg((const float2*) (gp + a.I + 64));
                         const float wt = rt->w[tile][t];
                         // fp16 operands: the fast exponential is far inside their rounding; the int8 mode follows the CPU engine
+                        constexpr bool EXACT = Q8 || WIDE;
                         float v[2][2];
-                        v[0][0] = g0.x / (1.f + (Q8 ? expf(-g0.x) : __expf(-g0.x))) * u0.x * wt;
-                        v[0][1] = g0.y / (1.f + (Q8 ? expf(-g0.y) : __expf(-g0.y))) * u0.y * wt;
-                        v[1][0] = g1.x / (1.f + (Q8 ? expf(-g1.x) : __expf(-g1.x))) * u1.x * wt;
-                        v[1][1] = g1.y / (1.f + (Q8 ? expf(-g1.y) : __expf(-g1.y))) * u1.y * wt;
+                        v[0][0] = g0.x / (1.f + (EXACT ? expf(-g0.x) : __expf(-g0.x))) * u0.x * wt;
+                        v[0][1] = g0.y / (1.f + (EXACT ? expf(-g0.y) : __expf(-g0.y))) * u0.y * wt;
+                        v[1][0] = g1.x / (1.f + (EXACT ? expf(-g1.x) : __expf(-g1.x))) * u1.x * wt;
+                        v[1][1] = g1.y / (1.f + (EXACT ? expf(-g1.y) : __expf(-g1.y))) * u1.y * wt;
                         #pragma unroll
                         for (int blk = 0; blk < 2; ++blk)
                         {
@@ -460,12 +462,12 @@ static void launch_dependent(Kern kern, int grid, const DecodeArgs& a, cudaStrea
     cudaLaunchKernelEx(&cfg, kern, a);
 }
 
-template <bool G, bool Q, bool DOWN, int KC>
+template <bool G, bool Q, bool DOWN, int KC, bool WIDE = false>
 static void launch_stream(int grid, const DecodeArgs& a, cudaStream_t st, bool dependent)
 {
     static DeviceOnce once;
-    if (once.first()) cudaFuncSetAttribute(decode_stream_kernel<G, Q, DOWN, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, StreamSmem::total);
-    launch_dependent(decode_stream_kernel<G, Q, DOWN, KC>, grid, a, st, dependent);
+    if (once.first()) cudaFuncSetAttribute(decode_stream_kernel<G, Q, DOWN, KC, Route, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, StreamSmem::total);
+    launch_dependent(decode_stream_kernel<G, Q, DOWN, KC, Route, WIDE>, grid, a, st, dependent);
 }
 
 }  // namespace

@@ -143,10 +143,45 @@ def test_wide_shapes(oracle, dev, H, I, group, R):
     assert errors(got, ref)[2] < NORM_REL_EXACT, errors(got, ref)
 
 
+@pytest.mark.parametrize("H,I", [(8192, 2048), (2048, 4096)])
+def test_wide_layers_silu_in_fp32(dev, H, I):
+    """Layers wider than 6144 x 2048 compute SiLU(g) * u in fp32 with the accurate exponential. One code of 1 per row of each matrix makes every sum
+    one term and every fp16-rounded product visible: it is the rounding of the value in 64 bits wherever that lies farther from a boundary than
+    the fp32 arithmetic can move it (exponential, sum, quotient and two products, one unit in the last place each; one more for good measure). Gates around
+    -70, where an exponential that is off by half a unit per unit of its argument misses some of them."""
+    import torch
+    from hecate_b200 import layout, moe
+    rng = np.random.default_rng(H)
+    R, n = 16, min(H, I)                                      # n products of every row can be seen
+    def pick(N, K):
+        c = np.full((N, K), 8, dtype=np.uint8)
+        c[np.arange(N), np.arange(N) % K] = 9
+        return torch.from_numpy(layout.pack_u4(c)).to(dev)
+    x = rng.uniform(0.97, 1.0, (R, H)).astype(np.float16)
+    xk = x[:, np.arange(I) % H].astype(np.float32)
+    gs = rng.uniform(-85.0, -60.0, I).astype(np.float32)
+    us = (rng.uniform(0.5, 2.0, I) * np.exp(-gs.astype(np.float64)) / gs).astype(np.float32)
+    g, u = (xk * gs).astype(np.float64), (xk * us).astype(np.float64)          # the fp32 products the kernel forms
+    exact = (g / (1.0 + np.exp(-g)) * u)[:, :n]
+    up = lambda a: torch.from_numpy(a).to(dev)
+    tabs = moe.ExpertTables(H, I, 8, [pick(I, H)], [pick(I, H)], [pick(H, I)], [up(gs)], [up(us)], [torch.ones(H, device=dev)], device=dev)
+    sel = torch.full((R, 8), 99, dtype=torch.int64, device=dev); sel[:, 0] = 0
+    y, ws = torch.zeros(R, H, device=dev), moe.decode_workspace(H, I, dev)
+    moe.decode(tabs, up(x), sel, torch.ones(R, 8, dtype=torch.float16, device=dev), y, ws)
+    assert moe.ws_status(ws) == 0
+    got = y[:, :n].cpu().numpy().astype(np.float64)
+    margin = np.abs(exact) * 6 * 2.0 ** -23
+    below, above = (exact - margin).astype(np.float16), (exact + margin).astype(np.float16)
+    sure = below == above
+    assert sure.mean() > 0.99 and exact.min() > 2.0 ** -14 and exact.max() < 60000
+    off = np.count_nonzero(got[sure] != below[sure].astype(np.float64))
+    assert off == 0, (off, np.count_nonzero(sure))
+
+
 @pytest.mark.parametrize("H,I", [(6272, 256), (512, 2176)])
 def test_shapes_beyond_the_register_resident_path(oracle, dev, H, I):
-    """H > 6144 or I > 2048: a tile's activation fragments no longer fit in registers and the call takes the kernels that
-    fetch them stage by stage."""
+    """H > 6144 or I > 2048 in the int8 mode: a tile's activation fragments and scales no longer fit in registers and the call takes the kernels
+    that fetch them stage by stage."""
     (got,), ref = run_case(oracle, dev, H, I, 8, 11, 128, True, True, seed=5)
     assert int8_close(errors(got, ref)), errors(got, ref)
 
@@ -162,11 +197,12 @@ def test_wide_shapes_with_several_items_per_block(oracle, dev, H, I, aq):
             assert int8_close(e) if aq else e[2] < NORM_REL_EXACT, (group, e)
 
 
-@pytest.mark.parametrize("R,H,I,E,aq", [(16, 6144, 2048, 32, False), (5, 6144, 2048, 32, True), (1, 512, 256, 32, True), (13, 1024, 256, 64, False)])
+@pytest.mark.parametrize("R,H,I,E,aq", [(16, 6144, 2048, 32, False), (5, 6144, 2048, 32, True), (1, 512, 256, 32, True), (13, 1024, 256, 64, False),
+                                           (6, 7168, 2560, 32, False), (16, 8192, 384, 64, False), (3, 512, 4096, 32, False)])
 def test_router_decode_in_one_call_equals_the_two_calls(oracle, dev, R, H, I, E, aq):
     """hmoe_router_decode (the router's launch also does the decode call's set-up step) against hmoe_router followed by
     hmoe_decode: the same selection and weights bit for bit, the same output up to the order of the fp32 atomic additions; and
-    against the CPU checker."""
+    against the CPU checker. The second workspace has served other selections before."""
     import torch
     from hecate_b200 import moe
     hl = HostLayer(9, 0, H, I, range(E), 128, True)
@@ -181,6 +217,8 @@ def test_router_decode_in_one_call_equals_the_two_calls(oracle, dev, R, H, I, E,
     moe.router_fused(xt, wt, bias, None, None, sel1, rw1, 8, 1.5)
     moe.decode(tabs, xt, sel1, rw1, y1, ws, act_quant=aq)
     ws2 = moe.decode_workspace(H, I, dev)
+    sel2 = torch.empty(16, 8, dtype=torch.int64, device=dev); rw2 = torch.empty(16, 8, dtype=torch.float16, device=dev)
+    moe.router_decode(tabs, torch.randn(16, H, device=dev).to(torch.bfloat16), wt, bias, sel2, rw2, 1.5, torch.zeros(16, H, device=dev), ws2, act_quant=aq)
     for _ in range(2):                                        # twice: the counters inside the library return to zero
         sel2 = torch.full((R, 8), -7, dtype=torch.int64, device=dev); rw2 = torch.zeros(R, 8, dtype=torch.float16, device=dev)
         y2 = torch.zeros(R, H, device=dev)
