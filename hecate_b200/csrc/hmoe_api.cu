@@ -228,11 +228,14 @@ int hmoe_short_prefill_ep(const hmoe_layer* layer, const void* x, int x_dtype, c
 //   4096 x 1024, 128 experts: 64 rows 202 / 213, 128 rows 285 / 238;  int4 shared, 6144 x 2048, 256 experts: 160 rows 1023 / 954, 256 rows 1478 / 992
 // So the GEMMs take over once the tiles beyond the first of each expert, with the shared expert's, outweigh both: a block of the GEMMs
 // costs 1.10 tiles, the 40 us are 11 tiles of 6144 x 2048, and the int8 shared expert adds about half a
-// tile per row to the short path. The selections are not known here: the tiles are counted for picks spread evenly over 256 router positions, the
-// most there can be, so a call whose experts get more picks than that keeps the short path for longer than it should, never the reverse. The int8
+// tile per row to the short path. The selections are not known here. From position 0 on, the experts are taken for the layer's whole set, or its
+// first band, and the tiles beyond the first counted for picks spread evenly over 256 router positions: a smaller layer gets more
+// picks per expert than that and keeps the short path for longer than it should, and an uneven spread has more tiles still. A band further up may hold the
+// layer's rarely picked experts, and then has hardly a second tile (6144 x 2048, 64 of 256 experts, Zipf(1.3): 256 rows 199 / 230), so only what is certain
+// counts, the shared expert's tiles. The int8
 // activation mode walks the GEMMs' weights twice and keeps the plain limit. So do layers with scale groups: the short path applies the scales to fp32 sums, the
 // GEMMs to the fp16 weights, which is exact only from 2^-17 to below 8192.
-static bool gemms_win(const hmoe_layer* L, int R, int n_local, bool sh8)
+static bool gemms_win(const hmoe_layer* L, int R, int lo, int n_local, bool sh8)
 {
     if (n_local < 1 || L->group) return false;              // the GEMMs want experts
     const double n = n_local, m = (double) R * L->topk / 256.0;
@@ -240,14 +243,14 @@ static bool gemms_win(const hmoe_layer* L, int R, int n_local, bool sh8)
     for (int c = 0; c <= 40; ++c, p *= m / c) { cum += p; if (c && c % 8 == 0) extra += 1.0 - cum; }
     const double shared = L->sh_gate_w == nullptr ? 0.0 : sh8 ? 0.47 * R : R / 8.0;
     const double fixed = 11.0 * (6144.0 * 2048.0) / ((double) L->H * L->I);
-    return extra * n + shared > 0.10 * n + fixed;
+    return (lo == 0 ? extra * n : 0.0) + shared > 0.10 * n + fixed;
 }
-static int forward_path(const hmoe_layer* L, int R, int n_local, int act_quant)
+static int forward_path(const hmoe_layer* L, int R, int lo, int n_local, int act_quant)
 {
     const bool sh8 = L->shared_format == 1 && L->sh_gate_w != nullptr;
     if (sh8 && act_quant) return 2;           // the int8 shared expert in the int8 activation mode: only the grouped GEMMs serve it
     if (R <= MAXR) return 0;
-    if (R <= (sh8 ? FORWARD_SHORT_ROWS_SH8 : FORWARD_SHORT_ROWS) && L->I <= 2048 && L->H <= 6144 && (act_quant || !gemms_win(L, R, n_local, sh8))) return 1;
+    if (R <= (sh8 ? FORWARD_SHORT_ROWS_SH8 : FORWARD_SHORT_ROWS) && L->I <= 2048 && L->H <= 6144 && (act_quant || !gemms_win(L, R, lo, n_local, sh8))) return 1;
     return 2;
 }
 int hmoe_forward_short_rows(void) { return FORWARD_SHORT_ROWS; }
@@ -266,7 +269,7 @@ int hmoe_forward(const hmoe_layer* layer, const void* x, int x_dtype, const int6
     if (!layer) return fail(HMOE_E_ARG, "hmoe_forward: null layer");
     if (R < 1) return fail(HMOE_E_ARG, "hmoe_forward: rows must be >= 1");
     if (ws_bytes < hmoe_forward_ws_bytes(R, layer->topk, n_local, layer->H, layer->I, act_quant)) return fail(HMOE_E_WS, "hmoe_forward: workspace too small");
-    switch (forward_path(layer, R, n_local, act_quant))
+    switch (forward_path(layer, R, lo, n_local, act_quant))
     {
     case 0: return decode_launch(layer, x, x_dtype, sel, rw, R, lo, n_local, act_quant, out, ws, ws_bytes, (cudaStream_t) stream);
     case 1: return short_launch(layer, x, x_dtype, sel, rw, R, lo, n_local, act_quant, out, ws, ws_bytes, (cudaStream_t) stream);

@@ -261,14 +261,23 @@ def _forward_and_short(dev, tabs, g, R, E, lo, act):
     return got, want, launches
 
 
-@pytest.mark.parametrize("R,shared,lo,n,act", [(384, "int4", 0, 64, "bf16"), (300, "none", 0, 64, "fp16"), (260, "none", 32, 48, "bf16"),
-                                               (60, "int8", 0, 64, "fp16"), (384, "int4", 60, 9, "bf16")])
+@pytest.mark.parametrize("R,shared,lo,n,act", [(384, "int4", 0, 64, "bf16"), (300, "none", 0, 64, "fp16"), (60, "int8", 0, 64, "fp16"),
+                                               (384, "int4", 60, 9, "bf16"), (200, "int8", 128, 32, "bf16")])
 def test_forward_hands_over_to_the_grouped_gemms(dev, R, shared, lo, n, act):
     """Rows at which forward leaves the short path before its row limit (counted by the launches): the same result as the short path. Both
     round the SiLU product to fp16 once (2.8e-4 from the layer in 64 bits), so they differ by at most twice that."""
     tabs, _, g = _random_layer(dev, R, n, 0, shared)
     got, want, launches = _forward_and_short(dev, tabs, g, R, max(64, lo + n), lo, act)
     assert launches == 6                                    # permutation (3), gather, two GEMMs
+    assert float((got - want).double().norm() / want.double().norm()) < 5.6e-4
+
+
+@pytest.mark.parametrize("R,shared,lo,n", [(384, "none", 32, 48), (260, "none", 192, 64), (384, "none", 128, 128), (64, "int4", 32, 48)])
+def test_forward_keeps_bands_without_certain_tiles_on_the_short_path(dev, R, shared, lo, n):
+    """A band that does not start at position 0 may hold rarely picked experts: the GEMMs do not take over by an estimate of its picks."""
+    tabs, _, g = _random_layer(dev, R, n, 0, shared)
+    got, want, launches = _forward_and_short(dev, tabs, g, R, 256, lo, "bf16")
+    assert launches == 3                                    # set-up, gate / up, down
     assert float((got - want).double().norm() / want.double().norm()) < 5.6e-4
 
 
