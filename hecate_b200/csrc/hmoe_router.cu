@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(128, 3) router_tile_kernel(const uint16_t* __r
     }
     // lane l is left with values 2 l and 2 l + 1: row l / 4, experts 2 (l % 4) and + 1
     const int r = (warp & 1) * 8 + (lane >> 2), e = e0 + (warp >> 1) * 8 + 2 * (lane & 3);
-    if (r < nr) *(float2*) (logits + (size_t) (r0 + r) * E + e) = make_float2(v[0], v[1]);
+    if (r < nr) { float* l = logits + (size_t) (r0 + r) * E + e; l[0] = v[0]; l[1] = v[1]; }        // (the workspace need not be 8-byte aligned)
 }
 template <bool XBF, bool WBF>
 void launch_tile(cudaStream_t st, const uint16_t* x, const uint16_t* wt, int R, int H, int E, float* logits)

@@ -41,6 +41,25 @@ def test_router_bit_exact_tiled_rows(oracle, R, H, E, xbf, wbf):
     _run(oracle, R, H, E, 8, xbf, wbf, 0.05, 1.5, seed=R + H)
 
 
+@pytest.mark.parametrize("R", [4, 1025])
+def test_router_workspace_on_any_4_byte_boundary(R):
+    """hmoe_router only ever asked its workspace for the alignment of its words."""
+    import ctypes as C
+    import torch
+    from hecate_b200 import _lib, moe
+    dev, H, E = torch.device("cuda:0"), 512, 64
+    x, wt = torch.randn(R, H, device=dev).half(), torch.randn(E, H, device=dev).half()
+    n = moe.lib().hmoe_router_ws_bytes(C.c_int(R), C.c_int(E))
+    outs = []
+    for off in (0, 4):
+        ws = torch.zeros(n + 16, dtype=torch.uint8, device=dev)[off:]
+        sel, rw = torch.full((R, 8), -1, dtype=torch.int64, device=dev), torch.zeros(R, 8, dtype=torch.float16, device=dev)
+        _lib.check(moe.lib().hmoe_router(_lib.vp(x), C.c_int(_lib.F16), _lib.vp(wt), C.c_int(_lib.F16), None, C.c_int(R), C.c_int(H), C.c_int(E), C.c_int(8),
+                                         C.c_float(1.0), _lib.vp(sel), _lib.vp(rw), _lib.vp(ws), C.c_size_t(n), moe._stream(dev)))
+        outs.append((sel, rw))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1].view(torch.int16), outs[1][1].view(torch.int16)) and int(outs[0][0].min()) >= 0
+
+
 def test_router_large_rows(oracle):
     _run(oracle, 1000, 512, 128, 8, 1, 1, 0.05, 1.0, seed=9)
 
