@@ -636,11 +636,11 @@ static void launch_pair(int grid, const DecodeArgs& a, int R, cudaStream_t st)
     else if (a.H <= 2048) launch_stream<G, Q, false, 1>(grid, a, st, !g_prof);
     else if (a.H <= 4096) launch_stream<G, Q, false, 2>(grid, a, st, !g_prof);
     else if (a.H <= 6144) launch_stream<G, Q, false, 3>(grid, a, st, !g_prof);
-    else launch_wide_stream(G, false, grid, &a, st, !g_prof);
+    else launch_wide_stream(G, false, grid, a, st, !g_prof);
     if (g_prof) cudaEventRecord(ev[2], st);
     if (!resident) decode_down_kernel<G, Q><<<grid, NTHREADS, SmemLayout::total, st>>>(a, R);
     else if (a.I <= 2048 && a.H <= 6144) launch_stream<G, Q, true, 1>(grid, a, st, !g_prof);
-    else launch_wide_stream(G, true, grid, &a, st, !g_prof);
+    else launch_wide_stream(G, true, grid, a, st, !g_prof);
     if (g_prof) { cudaEventRecord(ev[3], st); ++g_prof_calls; }
 }
 

@@ -5,11 +5,6 @@
 #include "hmoe_internal.h"
 
 namespace hmoe {
-namespace {
-
-constexpr int CW = 16;                   // warps per block
-constexpr int NTHREADS = CW * 32;
-constexpr int NSTAGE = 3;
 
 // The expert-parallel combine, done by the down launch itself when its blocks run out of weights to stream (instead of a kernel
 // of its own after it). The block that finishes last raises this rank's generation in every peer's flag array (release, system
@@ -26,6 +21,30 @@ struct EpTail
     unsigned* done;                   // arrival counter of this launch's blocks (in the workspace, returns to zero)
     unsigned* status;                 // status word for a wait that gives up
 };
+
+struct DecodeArgs
+{
+    int H, I;
+    const int64_t* gate_w; const int64_t* up_w; const int64_t* down_w;
+    const int64_t* gate_s; const int64_t* up_s; const int64_t* down_s;
+    const void* sh_gw; const void* sh_uw; const void* sh_dw; const void* sh_gs; const void* sh_us; const void* sh_ds;
+    const Route* route;
+    const __half* xf;      // [R][H] prepared rows
+    const float* xscale;   // [R][H/32] (Q8)
+    __half* act;           // [tiles][8][I] gate_up output = down input
+    float* ascale;         // [tiles][8][I/32] (Q8)
+    float* G;              // register-resident path: [pick rows][gate | up][I] fp32 sums (shares memory with act)
+    float* y;              // [R][H] (expert-parallel: base of two slots, the step's slot is chosen by *gen_ptr & 1)
+    const unsigned* gen_ptr; size_t slot_stride;
+    unsigned* status;
+    EpTail ep;             // expert parallel: the combine over peer memory as the tail of the down launch (world = 0: none)
+};
+
+namespace {
+
+constexpr int CW = 16;                   // warps per block
+constexpr int NTHREADS = CW * 32;
+constexpr int NSTAGE = 3;
 
 __device__ __forceinline__ void ep_st_release_sys(unsigned* p, unsigned v) { asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
 __device__ __forceinline__ unsigned ep_ld_acquire_sys(const unsigned* p)
@@ -88,24 +107,6 @@ __device__ __forceinline__ void ep_tail_combine(const EpTail& e, unsigned gen, s
         *(float4*) (e.f + o) = acc;
     }
 }
-
-struct DecodeArgs
-{
-    int H, I;
-    const int64_t* gate_w; const int64_t* up_w; const int64_t* down_w;
-    const int64_t* gate_s; const int64_t* up_s; const int64_t* down_s;
-    const void* sh_gw; const void* sh_uw; const void* sh_dw; const void* sh_gs; const void* sh_us; const void* sh_ds;
-    const Route* route;
-    const __half* xf;      // [R][H] prepared rows
-    const float* xscale;   // [R][H/32] (Q8)
-    __half* act;           // [tiles][8][I] gate_up output = down input
-    float* ascale;         // [tiles][8][I/32] (Q8)
-    float* G;              // register-resident path: [pick rows][gate | up][I] fp32 sums (shares memory with act)
-    float* y;              // [R][H] (expert-parallel: base of two slots, the step's slot is chosen by *gen_ptr & 1)
-    const unsigned* gen_ptr; size_t slot_stride;
-    unsigned* status;
-    EpTail ep;             // expert parallel: the combine over peer memory as the tail of the down launch (world = 0: none)
-};
 
 // Two 64-column blocks (one scale group) of a 64-row group: 4 strips x 8 steps of MMAs on the tile, added into acc with
 // the scales applied. wsm = shared address of the first block's 2 KB unit; the second follows it.
@@ -203,7 +204,7 @@ struct StreamSmem
     static constexpr int total = flags + 16;
 };
 
-// WIDE: layers wider than 6144 x 2048, whose SiLU has always been computed with expf, as in the int8 mode.
+// WIDE: layers wider than 6144 x 2048, whose SiLU has always been computed with expf, as in the int8 mode, and which the fused combine does not serve.
 template <bool GROUPED, bool Q8, bool DOWN, int KC, typename RT = Route, bool WIDE = false>
 __global__ void __launch_bounds__(NTHREADS, 1) decode_stream_kernel(const DecodeArgs a)
 {
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) decode_stream_kernel(const Decode
     __syncthreads();
     abort_drain(abort_flag);
     TL_MAX(DOWN ? 9 : 1);
-    if (DOWN && a.ep.world > 0) ep_tail_combine(a.ep, *a.gen_ptr, a.slot_stride, a.H);
+    if (DOWN && !WIDE && a.ep.world > 0) ep_tail_combine(a.ep, *a.gen_ptr, a.slot_stride, a.H);
 }
 
 template <typename Kern>

@@ -3,9 +3,8 @@
 
 namespace hmoe {
 
-void launch_wide_stream(bool grouped, bool down, int grid, const void* args, cudaStream_t st, bool dependent)
+void launch_wide_stream(bool grouped, bool down, int grid, const DecodeArgs& a, cudaStream_t st, bool dependent)
 {
-    const DecodeArgs& a = *(const DecodeArgs*) args;
     if (!down) { if (grouped) launch_stream<true, false, false, 4>(grid, a, st, dependent); else launch_stream<false, false, false, 4>(grid, a, st, dependent); }
     else if (a.I > 2048) { if (grouped) launch_stream<true, false, true, 2, true>(grid, a, st, dependent); else launch_stream<false, false, true, 2, true>(grid, a, st, dependent); }
     else { if (grouped) launch_stream<true, false, true, 1, true>(grid, a, st, dependent); else launch_stream<false, false, true, 1, true>(grid, a, st, dependent); }

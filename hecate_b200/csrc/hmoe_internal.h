@@ -84,6 +84,8 @@ int permute_launch(const int64_t* sel, const void* rw, int R, int topk, int lo, 
                    int32_t* order, int32_t* tok, int32_t* eid, float* wt, int32_t* counts, int32_t* rbt, int32_t* plan2, void* ws, size_t ws_bytes,
                    cudaStream_t st);
 
-// hmoe_decode_wide.cu; args: a DecodeArgs
-void launch_wide_stream(bool grouped, bool down, int grid, const void* args, cudaStream_t st, bool dependent);
+struct DecodeArgs;            // hmoe_decode_stream.cuh
+// hmoe_decode_wide.cu
+void launch_wide_stream(bool grouped, bool down, int grid, const DecodeArgs& a, cudaStream_t st, bool dependent);
+
 }  // namespace hmoe
