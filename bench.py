@@ -564,7 +564,7 @@ def prefill_arm(args, dev, layer, torch, moe, synth, O, R=8192, zipf=1.1):
         "config": {"workload": f"prefill M={R} tokens, Zipf({zipf}) top-8 over {n_exp} experts + shared, H=6144, int4 g128 bf16 scales",
                    "l2": "inputs larger than L2 (4.85 GB of weights, 0.9 GB gathered inputs)", "max_picks_per_expert": int(counts.max()),
                    "min_picks_per_expert": int(counts.min())},
-        "roofline": {"bound": "tensor", "kernel": "prefill_gemm_kernel<2> + <1> (whole step: permute, gather, both grouped GEMMs)",
+        "roofline": {"bound": "tensor", "kernel": "prefill_gemm_kernel<false> + <true> (whole step: permute, gather, both grouped GEMMs)",
                      "achieved": tf, "peak": pk["bf16"], "unit": "TFLOP/s", "frac": tf / pk["bf16"], "peak_kind": pk["kind"] + " burst (bf16_tflops)",
                      "peak_sustained": pk["bf16_sustained"], "frac_sustained": tf / pk["bf16_sustained"], "traffic": None,
                      "algorithmic_flop_per_step": flop},

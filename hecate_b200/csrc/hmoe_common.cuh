@@ -272,12 +272,12 @@ using Route = RouteT<MAXT>;
 
 // Short prefill: more rows than a decode call takes, still so few that most experts see fewer than eight of them, so the
 // streaming kernels (every distinct expert read once at memory speed) beat the grouped tensor-core GEMMs (whose weight
-// conversion costs the same for a 3-pick row block as for a 256-pick one). The reference has the same range between its
+// conversion costs the same for a 3-pick row block as for a 60-pick one). The reference has the same range between its
 // decode and its grouped-GEMM paths (runtime/tier/tier_split.py:341-355: 9..64 rows through the moe4 decode kernels in 8-row
 // chunks, each chunk streaming its experts again); here the whole call is one tile list, so an expert is streamed once per
 // eight of its picks. A pick is one tile column (an expert picked twice by a row gets two columns of that row).
-constexpr int SHORT_MAXR = 640;               // where the grouped GEMMs catch up on a 256-expert layer under uniform routing (row numbers and the rows
-                                              // of the per-pick buffer are 16-bit in the route)
+constexpr int SHORT_MAXR = 640;               // row numbers and the rows of the per-pick buffer are 16-bit in the route; the grouped GEMMs are the faster
+                                              // ones well below it (256 experts of 6144 x 2048, uniform routing: from about 230 rows on)
 // tiles: one partial tile per local expert and for the shared expert, plus the full ones
 constexpr int SHORT_MAXT = 256 + 1 + (SHORT_MAXR * TOPK_MAX) / 8 + SHORT_MAXR / 8 + 2;
 using RouteShort = RouteT<SHORT_MAXT, unsigned short>;

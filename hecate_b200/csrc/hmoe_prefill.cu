@@ -23,17 +23,17 @@
 //              act = SiLU(g) * u * routing weight in fp16; down adds scale * sum into out[token] with coalesced fp32 reductions.
 // What bounds it: up to about 64 picks per expert HBM (every expert's codes once), next to it the conversion (a code costs two of
 // the half-rate instructions, whatever the number of picks); from there on the tensor core at the clock the power cap leaves.
-// Measured (256 experts of 6144 x 2048, us per call before -> after, before: fp16 weights staged through shared memory, row blocks of up
-// to 256 picks): 777 rows, Zipf(1.1) 2872 -> 1735; 2048 rows, fp32 row scales 2753 -> 1821; 8192 rows, Zipf(1.1) 6821 -> 6416 (the last two at
-// 1.45 GHz under the power cap).
+// Measured, 256 experts of 6144 x 2048, us per call on new inputs: 777 rows, Zipf(1.1) 1713; 2048 rows, fp32 row scales 1758; 8192 rows, Zipf(1.1) 6178 (the
+// last two at 1.45 GHz under the power cap). With fp16 weights staged through shared memory and row blocks of up to 256 picks: 2874, 2825 and
+// 6971. Experts of 150 to 256 picks were converted once there and twice here, which a layer of few experts pays for (1500 rows over 64
+// experts of 8192 x 1536, scale groups: 1110 there, 1165 here).
 // The converting warps' issue slots are what a stage of few picks waits for (measured alone, four warps on a scheduler: 280 cycles per 16 words
 // of group-scaled codes, 210 of plain ones; beside them eight MMAs of 16 picks take 1240 cycles to issue instead of 470), so all that is not
 // conversion is kept short: the stage's inputs count their bytes on the barrier that the MMA warps wait for, a group steps over the other
-// group's stages, and slots and parities follow from running numbers. moe.prefill on random picks, us before -> after: scale groups, 64 rows
-// 1075 -> 998, 256 rows 1296 -> 1210, 2048 rows 1850 -> 1775; row scales, 2048 rows 1808 -> 1627, 4096 rows 3170 -> 2900.
+// group's stages, and slots and parities follow from running numbers.
 // Blocks are persistent (one per SM) over (row block, channel tile) items, channel tile fastest, so the blocks working at
 // the same time share one input tile and one expert's weights through L2.
-// Every wait is bounded (see mbar_wait); tensor memory is released by the warp that allocated it on every path.
+// Every wait is bounded (see pf_wait); tensor memory is released by the warp that allocated it on every path.
 #include <cuda.h>
 #include <type_traits>
 #include "hmoe_common.cuh"
@@ -408,7 +408,7 @@ __device__ __forceinline__ void scale_pair(uint32_t bf2, uint32_t& s_lo, uint32_
 
 // shared memory: the packed codes (four 64-row x 128-column blocks of 4 KB and their scales) and the inputs (two 64-column tiles) of
 // the stages in flight. Codes are requested NCODE stages ahead (68 KB per SM: more than the 45 KB that cover a microsecond at the
-// memory's full rate; five or seven slots measured no faster), inputs NB stages ahead; the converted weights never come here.
+// memory's full rate; seven slots, with three for the inputs, measured no faster), inputs NB stages ahead; the converted weights never come here.
 struct PfSmem
 {
     static constexpr int NCODE = PF_NCODE, NB = 4;           // powers of two: a running stage number gives slot and parity

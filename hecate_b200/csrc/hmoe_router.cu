@@ -607,9 +607,12 @@ int router_launch(const void* x, int x_dtype, const void* wt, int w_dtype, const
     float* logits = (float*) ((char*) ws + 256);
     const uint16_t* xp = (const uint16_t*) x; const uint16_t* wp = (const uint16_t*) wt;
     // The tiled kernel costs about 4 us per 1024 columns however few the rows (25 us for 6144), the other one a wave of blocks per four rows x
-    // eight experts x resident blocks: measured, us, other / tiled, 6144 columns x 256 experts: 32 rows 23 / 25, 48 rows 29 / 25, 64 rows
-    // 37 / 25, 1024 rows 431 / 95; 2048 x 64 (three blocks per SM): 200 rows 14.5 / 16.9, 256 rows 20.3 / 16.9; 8192 x 32: 256 rows
-    // 27 / 29, 400 rows 39 / 29. So it takes over after two waves, or one where three or more blocks share an SM.
+    // eight experts x resident blocks. It takes over where the other one has more than max(2, blocks that fit an SM's shared memory) blocks per SM; with two
+    // fitting (2560 to 3584 columns) that is one full wave, with one fitting two waves. Measured, us, other / tiled, the first rows beyond the line: 6144 columns x
+    // 256 experts: 48 rows 29 / 25, 64 rows 37 / 25, 1024 rows 431 / 95; 3072 x 256: 36 rows 14.5 (before the line), 37 rows 19.2 / 16.6; 2560 x 32: 297
+    // rows 17.1 / 16.5; 2048 x 256: 53 rows 17.6 / 14.3; 8192 x 256: 37 rows 35 / 29. Of 168 points around the line, 256 to 8192 columns, none is
+    // slower than the other kernel. Up to 1024 columns the threads bound the blocks per SM and the line is later than it need be (256 x 256: 313
+    // rows 24.8 / 14.5).
     const int sms = device_sms();
     if (sms <= 0) return fail(HMOE_E_CUDA, "hmoe_router: no current CUDA device");
     const int per_sm = (int) (227u * 1024u / (smem + 1024)), waves = per_sm > 2 ? per_sm : 2;

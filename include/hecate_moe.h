@@ -172,7 +172,8 @@ int hmoe_permute(const int64_t* sel, const void* rw, int R, int topk, int lo, in
  * permute -> gather -> grouped gate+up GEMM with SiLU * up * weight epilogue -> grouped down GEMM whose epilogue adds
  * scale * sum into out[token] (fp32 [R][H], added into: zero it first for a plain result). tcgen05 tensor cores, fp16
  * operands, fp32 accumulation. Row scales are applied to the fp32 sums; group scales (group = 128) to the fp16 weights, exactly for scales from 2^-17 to
- * below 8192 in size (smaller ones lose bits, 8 x 8192 is infinite; hmoe_decode and hmoe_short_prefill apply them to fp32 sums). act_quant = 1 reproduces the CPU engine's int8 activation round trips: code x scale is carried
+ * below 8192 in size (smaller ones lose bits, 8 x 8192 is infinite; hmoe_decode and hmoe_short_prefill apply them to fp32 sums).
+ * act_quant = 1 reproduces the CPU engine's int8 activation round trips: code x scale is carried
  * as an fp16 hi + lo pair and the weights are walked twice (twice the tensor-core work; a parity mode, not the fast path).
  * Other arguments as hmoe_decode. ws: hmoe_prefill_ws_bytes(..., act_quant) bytes (holds the gathered inputs and the
  * intermediate activations: (R*topk + R) * (H + I) * 2 bytes, twice that in the int8 mode, plus small tables). */
@@ -184,7 +185,7 @@ int hmoe_prefill(const hmoe_layer* layer, const void* x, int x_dtype, const int6
  * runtime/tier/tier_split.py:341-355, that runs 9..64 rows through moe4.forward in 8-row chunks, each chunk streaming its
  * experts again). The whole call is one list of (expert, <= 8 picks) tiles for the decode streaming kernels, so a distinct
  * expert is read from memory once per eight of its picks; the grouped GEMMs convert every expert's weights whatever its row
- * count and only win from several hundred rows up (level at about 640 rows of uniform routing over 256 experts). Arguments as hmoe_prefill (out is added into). Needs H <= 6144, I <= 2048
+ * count and win from some 150 to 250 rows up (uniform routing over 256 experts, without the int8 shared expert). Arguments as hmoe_prefill (out is added into). Needs H <= 6144, I <= 2048
  * (else HMOE_E_UNSUPPORTED); the int8 shared expert runs sixteen rows at a time through the decode path's kernels and is not
  * available with act_quant = 1 (nor in hmoe_decode; hmoe_prefill and hmoe_forward serve that combination). ws: hmoe_short_prefill_ws_bytes(R, ...) bytes, 0 for R outside 1..640. */
 size_t hmoe_short_prefill_ws_bytes(int R, int H, int I, int topk);
@@ -199,7 +200,8 @@ int hmoe_short_prefill_ep(const hmoe_layer* layer, const void* x, int x_dtype, c
 /* One entry point for any number of rows, as tier_submit / _hot_prefill choose among the reference's kernels by row count
  * (runtime/tier/tier_split.py:341-364,543-546): R <= 16 -> hmoe_decode, then hmoe_short_prefill while it is
  * estimated to be the faster one (at most hmoe_forward_short_rows() rows, 256 with the int8 shared expert; when the layer's shapes allow it), else
- * hmoe_prefill. Layers with scale groups keep hmoe_short_prefill up to the row limit. The int8 shared expert with act_quant = 1 always takes hmoe_prefill. One workspace serves every row count up to
+ * hmoe_prefill. Layers with scale groups keep hmoe_short_prefill up to the row limit; of a band with lo > 0 only the shared expert's rows count.
+ * The int8 shared expert with act_quant = 1 always takes hmoe_prefill. One workspace serves every row count up to
  * the R it was sized for: hmoe_forward_ws_bytes(R_max, ...) bytes, zero-filled once. */
 int hmoe_forward_short_rows(void);
 size_t hmoe_forward_ws_bytes(int R, int topk, int n_local, int H, int I, int act_quant);
