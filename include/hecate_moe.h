@@ -248,8 +248,8 @@ int hmoe_ep_copy(void* dst, const void* src, size_t bytes, void* stream);
 /* The same two grouped GEMMs with the reference's calling convention, for callers that keep the reference's host-side
  * permutation: replaces moe4t.forward / moe4p.forward(x, tok, eid, wt, rbt, gw, uw, dw, gs, us, ds, gu, ar, d, out)
  * (runtime/tier/moe4/moe4t.cu:498-524). tok int32 [npos] (token of each sorted pick), wt fp32 [npos], rbt int32 [nrb][4] =
- * {expert, first pick, picks <= 256, 0}, all on the device; the expert of a pick is taken from its row block (eid is not
- * needed). Expert ids >= n_local select the shared expert. ws: hmoe_prefill_sorted_ws_bytes(npos, H, I) (replaces
+ * {expert, first pick, picks <= 256, 0} in any order, all on the device; the expert of a pick is taken from its row block (eid is not
+ * needed). Expert ids >= n_local select the shared expert, of either format. ws: hmoe_prefill_sorted_ws_bytes(npos, H, I) (replaces
  * moe4t.scratch, moe4t.cu:490-495). */
 size_t hmoe_prefill_sorted_ws_bytes(int npos, int H, int I, int act_quant);
 int hmoe_prefill_sorted(const hmoe_layer* layer, const void* x, int x_dtype, const int32_t* tok, const float* wt, const int32_t* rbt, int nrb,
